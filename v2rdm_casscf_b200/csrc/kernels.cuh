@@ -18,11 +18,16 @@ namespace v2g {
 extern std::atomic<long> g_kernel_launches;
 
 // A sparse map (A or A^T) in bucketed ELL form: rows are grouped by length
-// into buckets of fixed width (1, 2, 4, 8, 16, 32 slots, padding marked by
-// col = -1), stored slot-major so that a warp reads its table entries
+// into buckets of fixed width (1, 2, 4, 5, 8, 16, 32 slots, padding marked by
+// col = -1; the spin rows of A have five entries), stored slot-major so that a warp reads its table entries
 // coalesced and needs no row-pointer lookup; rows longer than 32 entries
-// (traces, contractions) are kept as CSR and reduced by a whole CTA each.
-constexpr int kMaxBuckets = 6;
+// (traces, contractions) are kept as CSR, the first nmid of them (at most
+// kMidRow entries, kMidMany or more rows of the same length) reduced by a warp
+// each, the others by a whole CTA.
+constexpr int kMaxBuckets = 7;
+constexpr int kMidRow = 256, kMidMany = 32;
+constexpr int kCodeShift = 27;                 // packed entry: 27 column bits, 4 code bits
+constexpr int kBookSize = 1 << (31 - kCodeShift);  // 16 coefficients at most
 struct DevMap {
     int64_t nrows = 0;  // output length
     int nb = 0;
@@ -31,15 +36,16 @@ struct DevMap {
     int64_t row_off[kMaxBuckets] = {};  // into rows
     int64_t ent_off[kMaxBuckets] = {};  // into cols / vals
     const int32_t* rows = nullptr;
-    // Entry words.  Unpacked: the column, with vals[] the coefficient.  Packed
-    // (book != nullptr, vals == nullptr): column | code << kCodeShift, the
-    // coefficient book[code] (the maps have a handful of distinct
-    // coefficients: +-1, +-1/2, -1/sqrt 2, a few small integers), 4 bytes per
-    // entry instead of 12.  Padding slots are -1 in both forms.
+    // Entry words.  Packed: column | code << kCodeShift, the coefficient
+    // book[code] (the maps have a handful of distinct coefficients: +-1,
+    // +-1/2, -1/sqrt 2, a few small integers), 4 bytes per entry instead of
+    // 12.  Unpacked (a table whose columns or coefficients do not fit): the
+    // column, with vals[] the coefficient.  Padding slots are -1 in both forms.
     const int32_t* cols = nullptr;
     const double* vals = nullptr;
-    const double* book = nullptr;
-    int nlong = 0;
+    int packed = 0;
+    double book[kBookSize] = {};
+    int nlong = 0, nmid = 0;
     const int32_t* long_rows = nullptr;
     const int32_t* long_ptr = nullptr;
     const int32_t* long_col = nullptr;
@@ -48,12 +54,9 @@ struct DevMap {
     // built-in rule); see kMapVariants
     int variant = -1;
 };
-constexpr int kCodeShift = 27;                 // packed entry: 27 column bits, 4 code bits
-constexpr int kBookSize = 1 << (31 - kCodeShift);  // 16 coefficients at most
-// Map kernel variants: instances per thread (2, 4, 8) and whether the table
-// loads and output stores bypass the caches (streaming hints).
-constexpr int kMapVariants = 4;  // 0: 2 plain, 1: 4 plain, 2: 4 streamed, 3: 8 streamed
-const char* map_variant_name(int v);
+// Map kernel variants: whether the table loads and output stores bypass the
+// caches (streaming hints).
+constexpr int kMapVariants = 2;  // 0: plain, 1: streamed
 
 // out[r,b] = coef[b] * (sum_k val[k] in[col[k],b] - sub[r]) + add[r,b]
 // (each of sub, coef, add optional); instances with mask[b] == 0 are skipped.

@@ -4,10 +4,12 @@
 // by all instances of a group (see kernels.cuh for the layouts).  A^T is
 // the transpose of A's table, so every primal element sums its contributing
 // constraints itself: no atomics, deterministic order, and the two maps are
-// exact adjoints.  These kernels are HBM-bound; their algorithmic traffic per
-// application is 8 * (dimx + nconstraints) bytes per instance.
+// exact adjoints.  The algorithmic traffic of an application is
+// 8 * (dimx + nconstraints) bytes per instance.
+#include <algorithm>
 #include <map>
 #include <mutex>
+#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -28,6 +30,9 @@ inline int grid_for(int64_t work, int threads = kThreads) {
 
 constexpr int kRedBlocks = 148 * 4;
 constexpr int kSpmvBlocks = 148 * 64;
+// resident CTAs of the map kernels (64 registers a thread; three CTAs with 80
+// registers: 334 us where four took 319, n = 20, 19 instances)
+constexpr int kMapCtasPerSm = 4;
 
 // Thread mapping shared by the map and vector kernels that also reduce: the
 // rows are cut into passes of T/B rows; pass k goes to block k % G, where
@@ -89,235 +94,408 @@ __device__ __forceinline__ void block_partial(double v, int B, double* __restric
     if ((int)threadIdx.x < B) partial[slot * B + threadIdx.x] = s;
 }
 
-// Per-row epilogue shared by the map kernels.
-struct Epi {
+// ---- the map kernels ---------------------------------------------------------
+//
+// Lanes run along the instances of a row: each of its lanes_of(B) lanes serves
+// one instance (B = 1) or two, so that a warp's gather of one table entry
+// reads B contiguous doubles per row, and the lanes of one row read the same
+// table entry (a broadcast).  With one row per lane and a chunk of instances
+// per thread, as before, every lane of every 8-byte load touched its own cache
+// line, and the L1 serves one line per clock.  What bounds the kernels now is
+// the latency of the chain table entry -> gather -> store (at one small
+// instance, beside the launch) and, in a batch, that latency against the loads
+// in flight.  In the deep form a thread works on several rows at once, a pass
+// of blockDim / lanes rows apart, with eight gathers in flight, and loads the
+// table entries of its next tile meanwhile.  The sum of a row runs in slot
+// order in one thread, whatever the form.  A and A^T one after the other on a
+// B200, before and now:
+//   n = 20, 19 instances   706 -> 275 us   (1.3 -> 3.4 TB/s of vector bytes)
+//   n = 28, 1 instance     243 ->  83 us
+//   n = 8 T2, 3 instances   99 ->  37 us
+//   n = 10, 1 instance     11.6 -> 9.8 us
+constexpr int kWarps = kThreads / 32;
+
+// How instances map to lanes: one lane each (B = 1), or two instances per
+// lane: l and l + (B + 1) / 2 for odd B (contiguous 8-byte loads), 2 l and
+// 2 l + 1 for even B (16-byte loads).
+enum LaneMode { kOne = 0, kOdd = 1, kEven = 2 };
+__host__ __device__ constexpr int lanes_of(int B) { return (B + 1) / 2; }
+static LaneMode lane_mode(int B) { return B == 1 ? kOne : ((B & 1) ? kOdd : kEven); }
+
+// Work units of one map application: first the long rows (a CTA each), then
+// the mid rows (a warp each, 32 instances at a time), then the row tiles.
+// Unit u runs on CTA u % gridDim.x.
+struct Blocks {
+    int start[kMaxBuckets + 1];  // first unit of each bucket's row tiles; the last: the unit count
+    int mid;                     // first mid-row unit
+    int midchunks;               // instance chunks of 32 per group of mid rows
+    int deep;                    // the deep form: ell_depth(width) rows per thread
+};
+
+// Rows per thread of the deep form, by bucket width.
+__host__ __device__ constexpr int ell_depth(int W) { return W == 1 ? 4 : (W == 2 ? 2 : 1); }
+
+// One thread's place among the tiles of a bucket.
+struct Lane {
+    int B, b0, b1;   // instances of this lane (b1 >= B: none)
+    int rsub, rpp;   // its row within a pass, rows per pass
+    bool on0, on1;   // instances present and not masked
+};
+
+template <int MODE>
+__device__ __forceinline__ Lane lane_of(int B, const int* mask) {
+    Lane L;
+    const int n = lanes_of(B), l = (int)threadIdx.x % n;
+    L.B = B;
+    L.rpp = (int)blockDim.x / n;
+    L.rsub = (int)threadIdx.x / n;
+    L.b0 = MODE == kEven ? 2 * l : l;
+    L.b1 = MODE == kEven ? 2 * l + 1 : (MODE == kOdd ? l + n : B);
+    L.on0 = !mask || mask[L.b0];
+    L.on1 = MODE != kOne && L.b1 < B && (!mask || mask[L.b1]);
+    return L;
+}
+
+// Predicated loads without a branch around each (the compiler's form of a
+// conditional load costs more instructions than the load): p where ok, else
+// the default (-1, 0).  COH: through L2 (ld.global.cg), for vectors that other
+// CTAs of the same (persistent) launch write, never from a stale L1 line.
+template <bool STREAM>
+__device__ __forceinline__ int32_t load_word(const int32_t* p, bool ok) {
+    int32_t v;
+    if (STREAM)
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.s32 %0, -1;\n\t@q ld.global.cs.b32 %0, [%1];\n\t}"
+            : "=&r"(v)
+            : "l"(p), "r"((int)ok));
+    else
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.s32 %0, -1;\n\t@q ld.global.nc.b32 %0, [%1];\n\t}"
+            : "=&r"(v)
+            : "l"(p), "r"((int)ok));
+    return v;
+}
+template <bool COH>
+__device__ __forceinline__ double load_one(const double* p, bool ok) {
+    double v;
+    if (COH)
+        asm volatile(
+            "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+            "@q ld.global.cg.f64 %0, [%1];\n\t}"
+            : "=&d"(v)
+            : "l"(p), "r"((int)ok)
+            : "memory");
+    else
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+            "@q ld.global.nc.f64 %0, [%1];\n\t}"
+            : "=&d"(v)
+            : "l"(p), "r"((int)ok));
+    return v;
+}
+template <bool COH>
+__device__ __forceinline__ double2 load_two(const double* p, bool ok) {
+    double2 v;
+    if (COH)
+        asm volatile(
+            "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+            "mov.f64 %1, 0d0000000000000000;\n\t@q ld.global.cg.v2.f64 {%0, %1}, [%2];\n\t}"
+            : "=&d"(v.x), "=&d"(v.y)
+            : "l"(p), "r"((int)ok)
+            : "memory");
+    else
+        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+            "mov.f64 %1, 0d0000000000000000;\n\t@q ld.global.nc.v2.f64 {%0, %1}, [%2];\n\t}"
+            : "=&d"(v.x), "=&d"(v.y)
+            : "l"(p), "r"((int)ok));
+    return v;
+}
+
+// What happens to the sum s of row r for instance b.  The returned values are
+// summed per instance where kSum is set.
+
+// out = A in
+struct EpiStore {
+    static constexpr bool kSum = false;
+    double* out;
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t r, int B, int b, double s) const {
+        out[(int64_t)r * B + b] = s;
+        return 0.0;
+    }
+};
+// out = coef (A in - sub) + add, each part optional
+struct EpiAffine {
+    static constexpr bool kSum = false;
     const double* sub;
     const double* coef;
     const double* add;
+    double* out;
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t r, int B, int b, double s) const {
+        const int64_t t = (int64_t)r * B + b;
+        if (sub) s -= sub[r];
+        if (coef) s *= coef[b];
+        if (add) s += add[t];
+        out[t] = s;
+        return 0.0;
+    }
+};
+// out = A in, summing dotv . out
+struct EpiDot {
+    static constexpr bool kSum = true;
     const double* dotv;
     double* out;
-};
-// COH: the vectors are written by other CTAs of the same (persistent) launch,
-// so they are loaded through L2 (ld.global.cg), never from a stale L1 line.
-template <bool STREAM = false, bool COH = false>
-__device__ __forceinline__ double epilogue(const Epi& e, int64_t r, int B, int b, double s) {
-    const int64_t t = r * B + b;
-    if (e.sub) s -= e.sub[r];
-    if (e.coef) s *= e.coef[b];
-    if (e.add) s += e.add[t];
-    if (STREAM)
-        __stcs(e.out + t, s);  // written once, not read again by this launch
-    else
-        e.out[t] = s;
-    if (!e.dotv) return 0.0;
-    return (COH ? __ldcg(e.dotv + t) : e.dotv[t]) * s;
-}
-
-// Bucketed-ELL part.  One lane per row (slot index i of its bucket) and a
-// chunk of up to CH consecutive instances per thread: the table loads of a
-// warp are 32 consecutive slots (coalesced), and every thread keeps
-// W x (instances) independent gathers in flight.  The instances of a chunk are
-// adjacent in memory ([col * B + b0 .. b0 + cnt)), loaded as double2 when B is
-// even.  Per instance the entries are summed in slot order, so the result does
-// not depend on the chunking.  CH = 4 (80 registers, three CTAs per SM) was
-// the fastest of 2, 4 and 8 at n = 12..20 with 8..20 instances (B200); single
-// instances use CH = 2 (64 registers).
-constexpr int kSlotBatch = 4;  // slots whose gathers are issued together
-
-struct Blocks {
-    int start[kMaxBuckets + 1];  // first row tile of each bucket
-    int nchunk;                  // instance chunks per row tile
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t r, int B, int b, double s) const {
+        const int64_t t = (int64_t)r * B + b;
+        out[t] = s;
+        return (COH ? __ldcg(dotv + t) : dotv[t]) * s;
+    }
 };
 
-template <int W, bool VEC, int CH, bool STREAM, bool PK, bool COH>
-__device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int64_t tile0, int64_t ntile, int B, int b0,
-                                         int cnt, unsigned act, const double* __restrict__ in, const Epi& e,
-                                         const double* sbook, double (&dot)[CH]) {
-    constexpr int KB = W < kSlotBatch ? W : kSlotBatch;
-    const int64_t ns = M.nslots[bi];
+// The tiles t0, t0 + tstep, ... of bucket bi, whose width is 1, 2, 5 (WB) or a
+// multiple of four (WB = 4, nbatch batches of slots).  A bucket has fewer than
+// 2^32 table entries (the table has fewer than 2^31, and padding at most
+// doubles a row), so table offsets are 32-bit.
+template <int WB, int MODE, bool DEEP, bool STREAM, bool PK, bool COH, class Epi>
+__device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int nbatch, int t0, int tstep, const Lane& L,
+                                         const double* __restrict__ in, const Epi& e, const double* sbook,
+                                         double (&dot)[2]) {
+    constexpr int R = DEEP ? ell_depth(WB) : 1;
+    constexpr int32_t kCol = PK ? (1 << kCodeShift) - 1 : -1;
+    static_assert(!DEEP || PK, "the deep form reads packed tables");
+    const uint32_t ns = (uint32_t)M.nslots[bi];
     const int32_t* rows = M.rows + M.row_off[bi];
     const int32_t* cols = M.cols + M.ent_off[bi];
     const double* vals = PK ? nullptr : M.vals + M.ent_off[bi];
-    for (int64_t i = tile0 * kThreads + threadIdx.x; i < ns; i += ntile * kThreads) {
-        double acc[CH];
+    const char* in0 = reinterpret_cast<const char*>(in + L.b0);
+    const int sB = 8 * L.B, second = 8 * (L.b1 - L.b0);  // bytes between columns, between the lane's instances
+    const uint32_t rpp = (uint32_t)L.rpp;
+    // 64-bit, so that the position past the last tile cannot wrap around
+    int64_t i = (int64_t)t0 * L.rpp * R + L.rsub;
+    const int64_t step = (int64_t)tstep * L.rpp * R;
+    if (i >= ns) return;
+    auto load = [&](uint32_t at, uint32_t k0, bool any, int32_t (&w)[WB][R]) {
 #pragma unroll
-        for (int j = 0; j < CH; j++) acc[j] = 0.0;
+        for (int j = 0; j < R; j++)
 #pragma unroll
-        for (int k0 = 0; k0 < W; k0 += KB) {
-            int c[KB];
-            double v[KB];
+            for (int k = 0; k < WB; k++)
+                w[k][j] = load_word<STREAM>(cols + (size_t)((k0 + k) * ns + at + j * rpp), any && at + j * rpp < ns);
+    };
+    auto rowids = [&](uint32_t at, bool any, int32_t (&r)[R]) {
 #pragma unroll
-            for (int k = 0; k < KB; k++) {
-                const int32_t wd = STREAM ? __ldcs(cols + (int64_t)(k0 + k) * ns + i)
-                                          : __ldg(cols + (int64_t)(k0 + k) * ns + i);
-                if (PK) {
-                    c[k] = wd < 0 ? -1 : (wd & ((1 << kCodeShift) - 1));
-                    v[k] = sbook[wd < 0 ? 0 : (wd >> kCodeShift)];
-                } else {
-                    c[k] = wd;
-                    v[k] = STREAM ? __ldcs(vals + (int64_t)(k0 + k) * ns + i)
-                                  : __ldg(vals + (int64_t)(k0 + k) * ns + i);
+        for (int j = 0; j < R; j++) r[j] = load_word<STREAM>(rows + (size_t)(at + j * rpp), any && at + j * rpp < ns);
+    };
+    int32_t w[WB][R], r[R];
+    load((uint32_t)i, 0, true, w);
+    rowids((uint32_t)i, true, r);
+    while (true) {
+        const int64_t next = i + step;
+        const bool more = next < ns;
+        double a0[R], a1[R];
+        int32_t rn[R];
+#pragma unroll
+        for (int j = 0; j < R; j++) a0[j] = a1[j] = 0.0;
+#pragma unroll 1
+        for (int kb = 0; kb < (WB == 4 ? nbatch : 1); kb++) {
+            double g0[WB][R], g1[WB][R], v[WB][R];
+#pragma unroll
+            for (int k = 0; k < WB; k++)
+#pragma unroll
+                for (int j = 0; j < R; j++) {
+                    const bool ok = w[k][j] >= 0;
+                    const double* q = reinterpret_cast<const double*>(in0 + (int64_t)(w[k][j] & kCol) * sB);
+                    if (MODE == kEven) {
+                        const double2 t = load_two<COH>(q, ok);
+                        g0[k][j] = t.x;
+                        g1[k][j] = t.y;
+                    } else {
+                        g0[k][j] = load_one<COH>(q, ok);
+                        if (MODE == kOdd)
+                            g1[k][j] = load_one<COH>(
+                                reinterpret_cast<const double*>(reinterpret_cast<const char*>(q) + second),
+                                ok && L.b1 < L.B);
+                    }
+                    if (!PK)
+                        v[k][j] = load_one<false>(vals + (size_t)((kb * WB + k) * ns + (uint32_t)i + j * rpp), ok);
                 }
+            int32_t wn[WB][R];
+            if (WB == 4 && kb + 1 < nbatch) {
+                load((uint32_t)i, (kb + 1) * WB, true, wn);  // the next batch of slots
+            } else if (DEEP) {
+                load((uint32_t)next, 0, more, wn);  // the next tile's first
+                rowids((uint32_t)next, more, rn);
             }
 #pragma unroll
-            for (int k = 0; k < KB; k++) {
-                if (c[k] < 0) continue;
-                const double* g = in + (int64_t)c[k] * B + b0;
-                if (VEC) {
+            for (int k = 0; k < WB; k++)
 #pragma unroll
-                    for (int j = 0; j < CH; j += 2)
-                        if (j < cnt) {
-                            const double2 q = COH ? __ldcg(reinterpret_cast<const double2*>(g + j))
-                                                  : __ldg(reinterpret_cast<const double2*>(g + j));
-                            acc[j] += v[k] * q.x;
-                            acc[j + 1] += v[k] * q.y;
-                        }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < CH; j++)
-                        if (j < cnt) acc[j] += v[k] * (COH ? __ldcg(g + j) : __ldg(g + j));
+                for (int j = 0; j < R; j++) {
+                    // a padding slot adds 0 times some coefficient of the book
+                    const double c = PK ? sbook[(w[k][j] >> kCodeShift) & (kBookSize - 1)] : v[k][j];
+                    a0[j] += c * g0[k][j];
+                    if (MODE != kOne) a1[j] += c * g1[k][j];
+                    if (DEEP || WB == 4) w[k][j] = wn[k][j];
                 }
-            }
         }
-        const int64_t r = STREAM ? __ldcs(rows + i) : rows[i];
 #pragma unroll
-        for (int j = 0; j < CH; j++)
-            if (j < cnt && ((act >> j) & 1u)) dot[j] += epilogue<STREAM, COH>(e, r, B, b0 + j, acc[j]);
+        for (int j = 0; j < R; j++) {
+            if (r[j] >= 0) {
+                if (L.on0) dot[0] += e.template one<COH>(r[j], L.B, L.b0, a0[j]);
+                if (MODE != kOne && L.on1) dot[1] += e.template one<COH>(r[j], L.B, L.b1, a1[j]);
+            }
+            if (DEEP) r[j] = rn[j];
+        }
+        if (!more) break;
+        i = next;
+        if (!DEEP) {
+            load((uint32_t)i, 0, true, w);
+            rowids((uint32_t)i, true, r);
+        }
     }
 }
 
-// Instances [b0, b0 + cnt) of chunk ch: balanced, and in pairs when B is even
-// (so that double2 loads stay 16-byte aligned).
-__device__ __forceinline__ void chunk_range(int B, int nchunk, int ch, int& b0, int& cnt) {
-    if ((B & 1) == 0) {
-        const int P = B / 2;
-        b0 = 2 * (int)(((int64_t)ch * P) / nchunk);
-        cnt = 2 * (int)(((int64_t)(ch + 1) * P) / nchunk) - b0;
-    } else {
-        b0 = (int)(((int64_t)ch * B) / nchunk);
-        cnt = (int)(((int64_t)(ch + 1) * B) / nchunk) - b0;
+// Per-instance sums over the CTA (thread b < B gets instance b's) of a value
+// that warp w holds in lane l for instance c0 + l, l < cnt (0 elsewhere).
+__device__ __forceinline__ double warps_to_instances(double v, int c0, int cnt) {
+    __shared__ double sh[kWarps][32];
+    sh[threadIdx.x >> 5][threadIdx.x & 31] = v;
+    __syncthreads();
+    double t = 0.0;
+    const int l = (int)threadIdx.x - c0;
+    if (l >= 0 && l < cnt)
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += sh[w][l];
+    __syncthreads();
+    return t;
+}
+
+// Mid rows (33 to kMidRow entries): a warp per row and 32 instances; with
+// fewer than 17 instances the lanes also share the row's entries (lane l sums
+// entries l / B, l / B + 32 / B, ...) and fold by shuffles.  A CTA per row
+// (the long form) left the 5,792 such rows of A^T at n = 8 with T2 with 80
+// entries on 256 threads each (38 us of a 48 us launch at one instance).
+template <bool COH, class Epi>
+__device__ __forceinline__ double mid_rows(const DevMap& M, int B, const double* __restrict__ in, const Epi& e,
+                                           const int* __restrict__ mask, int group, int chunk) {
+    const int lane = threadIdx.x & 31;
+    const int m = group * (int)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int c0 = chunk * 32, cnt = B - c0 < 32 ? B - c0 : 32;
+    const int n = cnt <= 16 ? 32 / cnt : 1;
+    const int l = lane / cnt, b = c0 + lane % cnt;
+    double s = 0.0, res = 0.0;
+    if (m < M.nmid) {
+        const int k0 = M.long_ptr[m], k1 = M.long_ptr[m + 1];
+        if (l < n) {
+#pragma unroll 8
+            for (int k = k0 + l; k < k1; k += n) {
+                const double* g = in + (int64_t)__ldg(M.long_col + k) * B + b;
+                s += __ldg(M.long_val + k) * (COH ? __ldcg(g) : __ldg(g));
+            }
+        }
+        for (int left = n; left > 1;) {
+            const int h = (left + 1) / 2;
+            const double o = __shfl_down_sync(0xffffffffu, s, cnt * h);
+            if (l < left - h) s += o;
+            left = h;
+        }
+        if (lane < cnt && !(mask && !mask[b])) res = e.template one<COH>(M.long_rows[m], B, b, s);
     }
+    return res;
 }
 
 // Long rows: one CTA per row; thread t sums entries k = t / B, t / B + T / B,
-// ... for instance t % B, then a fixed-order reduction per instance.  Run by
-// the CTAs of ell_kernel past its row tiles (one launch per map).
-template <bool COH>
-__device__ __forceinline__ void long_row(const DevMap& M, int B, const double* __restrict__ in, const Epi& e,
-                                         const int* __restrict__ mask, double* __restrict__ partial,
-                                         int partial_base, int lr) {
-    __shared__ double shl[kThreads];
+// ... for instance t % B, then a fixed-order reduction per instance.
+template <bool COH, class Epi>
+__device__ __forceinline__ double long_row(const DevMap& M, int B, const double* __restrict__ in, const Epi& e,
+                                           const int* __restrict__ mask, int lr) {
     const int lanes = blockDim.x / B;
     const int b = threadIdx.x % B;
     const int l = threadIdx.x / B;
-    const int r = M.long_rows[lr];
     const int k0 = M.long_ptr[lr], k1 = M.long_ptr[lr + 1];
     double s = 0.0;
-    if (threadIdx.x < lanes * B)
+    if (l < lanes) {
+#pragma unroll 4
         for (int k = k0 + l; k < k1; k += lanes) {
-            const double* g = in + (int64_t)M.long_col[k] * B + b;
-            s += M.long_val[k] * (COH ? __ldcg(g) : *g);
+            const double* g = in + (int64_t)__ldg(M.long_col + k) * B + b;
+            s += __ldg(M.long_val + k) * (COH ? __ldcg(g) : __ldg(g));
         }
-    shl[threadIdx.x] = s;
-    __syncthreads();
+    }
+    const double t = cta_instance_sum(s, B);
     double acc = 0.0;
-    if (threadIdx.x < B) {
-        double t = 0.0;
-        for (int q = 0; q < lanes; q++) t += shl[threadIdx.x + q * B];
-        if (!(mask && !mask[threadIdx.x])) acc = epilogue<false, COH>(e, r, B, threadIdx.x, t);
-    }
-    __syncthreads();
-    if (partial) block_partial(threadIdx.x < B ? acc : 0.0, B, partial, (int64_t)partial_base + lr);
-    if (COH) __syncthreads();  // the shared partials are reused by the CTA's next unit
+    if ((int)threadIdx.x < B && !(mask && !mask[threadIdx.x]))
+        acc = e.template one<COH>(M.long_rows[lr], B, (int)threadIdx.x, t);
+    return acc;
 }
 
-// One row tile of an ELL bucket of width code wv (= 2 width + (B even)).
-template <int CH, bool STREAM, bool PK, bool COH>
-__device__ __forceinline__ void ell_tile(int wv, const DevMap& M, int bi, int64_t t0, int64_t nt, int B, int b0,
-                                         int cnt, unsigned act, const double* __restrict__ in, const Epi& e,
-                                         const double* sbook, double (&dot)[CH]) {
-#define V2G_ELL(W, V) ell_rows<W, V, CH, STREAM, PK, COH>(M, bi, t0, nt, B, b0, cnt, act, in, e, sbook, dot)
-    switch (wv) {
-        case 2: V2G_ELL(1, false); break;
-        case 3: V2G_ELL(1, true); break;
-        case 4: V2G_ELL(2, false); break;
-        case 5: V2G_ELL(2, true); break;
-        case 8: V2G_ELL(4, false); break;
-        case 9: V2G_ELL(4, true); break;
-        case 16: V2G_ELL(8, false); break;
-        case 17: V2G_ELL(8, true); break;
-        case 32: V2G_ELL(16, false); break;
-        case 33: V2G_ELL(16, true); break;
-        case 64: V2G_ELL(32, false); break;
-        default: V2G_ELL(32, true); break;
+// All the units of this CTA: returns to thread b < B the CTA's sum of the
+// optional dot for instance b (fixed order; 0 elsewhere).
+template <int MODE, bool DEEP, bool STREAM, bool PK, bool COH, class Epi>
+__device__ __forceinline__ double ell_cta(const DevMap& M, const Blocks& bl, int B, const double* __restrict__ in,
+                                          const Epi& e, const int* mask, const double* sbook) {
+    const int G = (int)gridDim.x;
+    double sum = 0.0;  // thread b: instance b
+    int u = (int)blockIdx.x;
+    for (; u < bl.mid; u += G) {
+        const double d = long_row<COH>(M, B, in, e, mask, M.nmid + u);
+        if (Epi::kSum) sum += d;
     }
-#undef V2G_ELL
+    for (; u < bl.start[0]; u += G) {
+        const int chunk = (u - bl.mid) % bl.midchunks, c0 = chunk * 32;
+        const double d = mid_rows<COH>(M, B, in, e, mask, (u - bl.mid) / bl.midchunks, chunk);
+        if (Epi::kSum) sum += warps_to_instances(d, c0, B - c0 < 32 ? B - c0 : 32);
+    }
+    const Lane L = lane_of<MODE>(B, mask);
+    double dot[2] = {0.0, 0.0};
+    if (L.rsub < L.rpp && (L.on0 || L.on1)) {
+#pragma unroll 1
+        for (int bi = 0; bi < M.nb; bi++) {
+            // the first unit of this bucket that is this CTA's
+            int t0 = ((int)blockIdx.x - bl.start[bi]) % G;
+            if (t0 < 0) t0 += G;
+            if (t0 >= bl.start[bi + 1] - bl.start[bi]) continue;
+            const int W = M.width[bi];
+            if (W == 1)
+                ell_rows<1, MODE, DEEP, STREAM, PK, COH>(M, bi, 1, t0, G, L, in, e, sbook, dot);
+            else if (W == 2)
+                ell_rows<2, MODE, DEEP, STREAM, PK, COH>(M, bi, 1, t0, G, L, in, e, sbook, dot);
+            else if (W == 5)
+                ell_rows<5, MODE, DEEP, STREAM, PK, COH>(M, bi, 1, t0, G, L, in, e, sbook, dot);
+            else
+                ell_rows<4, MODE, DEEP, STREAM, PK, COH>(M, bi, W / 4, t0, G, L, in, e, sbook, dot);
+        }
+    }
+    if (Epi::kSum) {
+        // two instances per lane: fold each half on its own, then to thread b
+        const int n = lanes_of(B);
+        const double s0 = cta_instance_sum(dot[0], n);
+        if (MODE == kOne) {
+            sum += s0;
+        } else {
+            __shared__ double sh[kThreads];
+            const double s1 = cta_instance_sum(dot[1], n);
+            if ((int)threadIdx.x < n) {
+                sh[MODE == kEven ? 2 * threadIdx.x : threadIdx.x] = s0;
+                const int b1 = MODE == kEven ? 2 * (int)threadIdx.x + 1 : (int)threadIdx.x + n;
+                if (b1 < B) sh[b1] = s1;
+            }
+            __syncthreads();
+            if ((int)threadIdx.x < B) sum += sh[threadIdx.x];
+            __syncthreads();
+        }
+    }
+    return sum;
 }
 
-// Work unit `blk` of one map application: a row tile of an ELL bucket times
-// an instance chunk (per-instance partial sums of the optional dot into
-// partial[tile * B + b]), or, past the tiles, one long row (its partial at
-// slot ntiles + row).  ell_kernel runs one unit per CTA; the persistent CG
-// kernel walks the units of a map with its whole grid (COH loads).
-template <int CH, bool STREAM, bool COH>
-__device__ __forceinline__ void ell_unit(const DevMap& M, const Blocks& bl, int B, const double* __restrict__ in,
-                                         const Epi& e, const int* mask, double* __restrict__ partial,
-                                         const double* sbook, int blk) {
-    const int ntiles = bl.start[M.nb];
-    if (blk >= ntiles * bl.nchunk) {
-        long_row<COH>(M, B, in, e, mask, partial, ntiles, blk - ntiles * bl.nchunk);
-        return;
-    }
-    const int tile = blk / bl.nchunk;
-    const int ch = blk % bl.nchunk;
-    int bi = 0;
-    while (bi + 1 < M.nb && tile >= bl.start[bi + 1]) bi++;
-    int b0, cnt;
-    chunk_range(B, bl.nchunk, ch, b0, cnt);
-    unsigned act = 0;
-    for (int j = 0; j < cnt; j++)
-        if (!mask || mask[b0 + j]) act |= 1u << j;
-    double dot[CH];
-#pragma unroll
-    for (int j = 0; j < CH; j++) dot[j] = 0.0;
-    if (act) {
-        const int64_t t0 = tile - bl.start[bi], nt = bl.start[bi + 1] - bl.start[bi];
-        const int wv = M.width[bi] * 2 + ((B & 1) == 0 ? 1 : 0);
-        if (M.book)
-            ell_tile<CH, STREAM, true, COH>(wv, M, bi, t0, nt, B, b0, cnt, act, in, e, sbook, dot);
-        else
-            ell_tile<CH, STREAM, false, COH>(wv, M, bi, t0, nt, B, b0, cnt, act, in, e, sbook, dot);
-    }
-    if (!partial) return;
-    // per-instance block sums in a fixed order: warp shuffles, then warps
-    __shared__ double sh[kThreads / 32][CH];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < CH; j++) {
-        double v = dot[j];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) sh[warp][j] = v;
-    }
-    __syncthreads();
-    if ((int)threadIdx.x < cnt) {
-        double t = 0.0;
-        for (int w = 0; w < kThreads / 32; w++) t += sh[w][threadIdx.x];
-        partial[(int64_t)tile * B + b0 + threadIdx.x] = t;
-    }
-    if (COH) __syncthreads();  // sh is reused by the CTA's next unit
-}
-
-template <int CH, bool STREAM>
-__global__ void __launch_bounds__(kThreads) ell_kernel(DevMap M, Blocks bl, int B, const double* __restrict__ in,
-                                                       Epi e, const int* __restrict__ mask,
-                                                       double* __restrict__ partial) {
+template <int MODE, bool DEEP, bool STREAM, bool PK, class Epi>
+__global__ void __launch_bounds__(kThreads, kMapCtasPerSm)
+    ell_kernel(const __grid_constant__ DevMap M, const __grid_constant__ Blocks bl, int B,
+               const double* __restrict__ in, const __grid_constant__ Epi e, const int* __restrict__ mask,
+               double* __restrict__ partial) {
     // the coefficient book of a packed table, in shared memory
     __shared__ double sbook[kBookSize];
-    if (M.book) {
+    if (PK) {
         if (threadIdx.x < kBookSize) sbook[threadIdx.x] = M.book[threadIdx.x];
         __syncthreads();
     }
-    ell_unit<CH, STREAM, false>(M, bl, B, in, e, mask, partial, sbook, blockIdx.x);
+    const double s = ell_cta<MODE, DEEP, STREAM, PK, false>(M, bl, B, in, e, mask, sbook);
+    if (Epi::kSum && (int)threadIdx.x < B) partial[(int64_t)blockIdx.x * B + threadIdx.x] = s;
 }
 
 // Stage 1: block g reduces a contiguous chunk of elements for every instance;
@@ -738,12 +916,12 @@ constexpr int kLoopCtasPerSm = 3;
 
 struct CgLoopArgs {
     DevMap A, AT;
-    Blocks blA, blAT;  // unit layouts of the two maps for ell_unit<CH, false>
+    Blocks blA, blAT;  // unit layouts of the two maps
     int B;
     int64_t nc;
     double *y, *r, *p, *atp, *ap;
     CgScalars* cs;
-    double* part_dot;  // (A's row tiles + long rows) x B
+    double* part_dot;  // grid x B
     double* part_rr;   // grid x B
     unsigned int* bar;
     int* err;
@@ -805,8 +983,8 @@ __device__ __forceinline__ void loop_reduce(const double* part, int n, int B, do
     __syncthreads();
 }
 
-template <int CH>
-__global__ void __launch_bounds__(kThreads, kLoopCtasPerSm) cg_loop_kernel(const CgLoopArgs L) {
+template <int MODE, bool DEEP, bool PK>
+__global__ void __launch_bounds__(kThreads, kLoopCtasPerSm) cg_loop_kernel(const __grid_constant__ CgLoopArgs L) {
     __shared__ double bookA[kBookSize], bookAT[kBookSize];
     __shared__ CgScalars sc[kLoopMaxB];
     __shared__ int sact[kLoopMaxB];
@@ -814,8 +992,8 @@ __global__ void __launch_bounds__(kThreads, kLoopCtasPerSm) cg_loop_kernel(const
     __shared__ int s_any;
     const int B = L.B;
     if (threadIdx.x < kBookSize) {
-        if (L.A.book) bookA[threadIdx.x] = L.A.book[threadIdx.x];
-        if (L.AT.book) bookAT[threadIdx.x] = L.AT.book[threadIdx.x];
+        bookA[threadIdx.x] = L.A.book[threadIdx.x];
+        bookAT[threadIdx.x] = L.AT.book[threadIdx.x];
     }
     if ((int)threadIdx.x < B) {
         sc[threadIdx.x] = L.cs[threadIdx.x];
@@ -824,11 +1002,8 @@ __global__ void __launch_bounds__(kThreads, kLoopCtasPerSm) cg_loop_kernel(const
     __syncthreads();
     const unsigned int G = gridDim.x;
     unsigned int target = 0;
-    const int unitsAT = L.blAT.start[L.AT.nb] * L.blAT.nchunk + L.AT.nlong;
-    const int unitsA = L.blA.start[L.A.nb] * L.blA.nchunk + L.A.nlong;
-    const int slotsA = L.blA.start[L.A.nb] + L.A.nlong;  // partial slots of the A map
-    const Epi eAT{nullptr, nullptr, nullptr, nullptr, L.atp};
-    const Epi eA{nullptr, nullptr, nullptr, L.p, L.ap};
+    const EpiStore eAT{L.atp};
+    const EpiDot eA{L.p, L.ap};
     int it = 0;
     while (true) {
         if (threadIdx.x == 0) {
@@ -839,16 +1014,17 @@ __global__ void __launch_bounds__(kThreads, kLoopCtasPerSm) cg_loop_kernel(const
         __syncthreads();
         if (!s_any || it >= L.cap) break;
         // A^T p
-        for (int u = blockIdx.x; u < unitsAT; u += G)
-            ell_unit<CH, false, true>(L.AT, L.blAT, B, L.p, eAT, sact, nullptr, bookAT, u);
+        ell_cta<MODE, DEEP, false, PK, true>(L.AT, L.blAT, B, L.p, eAT, sact, bookAT);
         target += G;
         if (!grid_wait(L.bar, target, L.err)) return;
         // Ap = A (A^T p) and the partials of p.Ap
-        for (int u = blockIdx.x; u < unitsA; u += G)
-            ell_unit<CH, false, true>(L.A, L.blA, B, L.atp, eA, sact, L.part_dot, bookA, u);
+        {
+            const double s = ell_cta<MODE, DEEP, false, PK, true>(L.A, L.blA, B, L.atp, eA, sact, bookA);
+            if ((int)threadIdx.x < B) L.part_dot[(int64_t)blockIdx.x * B + threadIdx.x] = s;
+        }
         target += G;
         if (!grid_wait(L.bar, target, L.err)) return;
-        loop_reduce(L.part_dot, slotsA, B, spap);
+        loop_reduce(L.part_dot, (int)G, B, spap);
         // y += alpha p, r -= alpha Ap (cg_solver.cc:159-165), partials of r.r
         {
             const int rpp = kThreads / B, lanes = rpp * B;
@@ -910,71 +1086,86 @@ static int spmv_grid(int64_t nrows, int B) {
     return (int)(g < 1 ? 1 : g);
 }
 
-// Row tiles (kThreads slots each) per ELL bucket, proportional to its slots,
-// at most kSpmvBlocks tiles in all; every tile runs once per instance chunk.
-const char* map_variant_name(int v) {
-    static const char* names[kMapVariants] = {"2 instances/thread", "4 instances/thread",
-                                              "4 instances/thread, streamed", "8 instances/thread, streamed"};
-    return (v >= 0 && v < kMapVariants) ? names[v] : "built-in rule";
+// Whether table loads and output stores bypass the caches (streaming hints):
+// the autotuner's choice, or streamed from eight instances up.
+static bool map_streamed(const DevMap& M, int B) {
+    if (M.variant >= 0 && M.variant < kMapVariants) return M.variant == 1;
+    return B >= 8;
 }
 
-static int map_variant(const DevMap& M, int B) {
-    if (M.variant >= 0 && M.variant < kMapVariants) return M.variant;
-    return B <= 2 ? 0 : (B < 8 ? 1 : 2);
+// CTA size for B instances: whole passes of a row's lanes, rounded up to
+// warps, and at least B (the per-instance sums end in thread b < B).
+static int map_threads(int B) {
+    const int n = lanes_of(B);
+    return std::max(kThreads / n * n, B) + 31 & ~31;
 }
 
-static Blocks map_blocks(const DevMap& M, int B) {
+// Units of a map (Blocks).  Small maps (every tile resident at once with one
+// row per thread) keep one row per thread: there the kernel is one latency
+// chain, and more CTAs spread it wider.
+static Blocks map_blocks(const DevMap& M, int B, int threads) {
     Blocks bl{};
-    const int var = map_variant(M, B);
-    const int ch = var == 0 ? 2 : (var == 3 ? 8 : 4);
-    bl.nchunk = (B + ch - 1) / ch;
+    const int64_t rpp = threads / lanes_of(B);
+    auto tiles = [&](int i, bool deep) {
+        const int64_t per = rpp * (deep ? ell_depth(M.width[i]) : 1);
+        return (M.nslots[i] + per - 1) / per;
+    };
     int64_t tot = 0;
-    for (int i = 0; i < M.nb; i++) tot += (M.nslots[i] + kThreads - 1) / kThreads;
-    const double scale = tot > kSpmvBlocks ? (double)kSpmvBlocks / (double)tot : 1.0;
-    int acc = 0;
+    for (int i = 0; i < M.nb; i++) tot += tiles(i, false);
+    bl.deep = M.packed && tot > 148 * kMapCtasPerSm;
+    bl.mid = M.nlong - M.nmid;
+    bl.midchunks = (B + 31) / 32;
+    const int warps = threads / 32;
+    int acc = bl.mid + (M.nmid + warps - 1) / warps * bl.midchunks;
     for (int i = 0; i < M.nb; i++) {
         bl.start[i] = acc;
-        int64_t g = (int64_t)(((M.nslots[i] + kThreads - 1) / kThreads) * scale);
-        if (g < 1) g = 1;
-        acc += (int)g;
+        acc += (int)tiles(i, bl.deep != 0);
     }
-    bl.start[M.nb] = acc;
+    for (int i = M.nb; i <= kMaxBuckets; i++) bl.start[i] = acc;
     return bl;
 }
 
-static int run_map(const DevMap& M, int B, const double* in, double* out, const double* sub, const double* coef,
-                   const double* add, const int* mask, const double* dotv, double* partial, cudaStream_t s) {
-    Epi e{sub, coef, add, dotv, out};
-    const Blocks bl = map_blocks(M, B);
-    if (M.nb > 0 || M.nlong > 0) {
-        // one launch: the row tiles of the ELL buckets (times the instance
-        // chunks), then one CTA per long row.  Variants: with 8 or more
-        // instances the table loads and the output stores are streamed past
-        // L1/L2 (cache-streaming hints), leaving the caches to the gathered
-        // input (7 % faster at n = 17..20 on B200, slower for single
-        // instances); the autotuner of each layout group picks per map
-        const int g = bl.start[M.nb] * bl.nchunk + M.nlong;
-        switch (map_variant(M, B)) {
-            case 0: ell_kernel<2, false><<<g, kThreads, 0, s>>>(M, bl, B, in, e, mask, partial); break;
-            case 1: ell_kernel<4, false><<<g, kThreads, 0, s>>>(M, bl, B, in, e, mask, partial); break;
-            case 2: ell_kernel<4, true><<<g, kThreads, 0, s>>>(M, bl, B, in, e, mask, partial); break;
-            default: ell_kernel<8, true><<<g, kThreads, 0, s>>>(M, bl, B, in, e, mask, partial); break;
-        }
-        g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+// Returns the partial sums written per instance (one per CTA, where the
+// epilogue sums).
+template <class Epi>
+static int run_map(const DevMap& M, int B, const double* in, const Epi& e, const int* mask, double* partial,
+                   cudaStream_t s) {
+    const int threads = map_threads(B);
+    const Blocks bl = map_blocks(M, B, threads);
+    const int units = bl.start[kMaxBuckets];
+    if (units == 0) return 0;
+    // as many CTAs as fit on the device at once, each with its share of the units
+    const int g = std::min(units, 148 * kMapCtasPerSm);
+    const bool st = map_streamed(M, B);
+    auto go = [&](auto mode) {
+        constexpr int MODE = decltype(mode)::value;
+        auto k = bl.deep ? (st ? ell_kernel<MODE, true, true, true, Epi> : ell_kernel<MODE, true, false, true, Epi>)
+                         : (M.packed ? ell_kernel<MODE, false, false, true, Epi>
+                                     : ell_kernel<MODE, false, false, false, Epi>);
+        k<<<g, threads, 0, s>>>(M, bl, B, in, e, mask, partial);
+    };
+    switch (lane_mode(B)) {
+        case kOne: go(std::integral_constant<int, kOne>()); break;
+        case kOdd: go(std::integral_constant<int, kOdd>()); break;
+        default: go(std::integral_constant<int, kEven>()); break;
     }
-    return bl.start[M.nb] + M.nlong;  // partial blocks written
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    return g;
 }
 
 void launch_spmv(const DevMap& A, int B, const double* in, double* out, const double* sub, const double* coef,
                  const double* add, const int* mask, cudaStream_t s) {
-    run_map(A, B, in, out, sub, coef, add, mask, nullptr, nullptr, s);
+    if (sub || coef || add)
+        run_map(A, B, in, EpiAffine{sub, coef, add, out}, mask, nullptr, s);
+    else
+        run_map(A, B, in, EpiStore{out}, mask, nullptr, s);
 }
 
 int64_t reduce_partial_size(int B) { return (int64_t)kSpmvBlocks * B; }
 
 void launch_spmv_dot(const DevMap& A, int B, const double* in, double* out, const double* dotv, const int* mask,
                      double* partial, double* dot_out, cudaStream_t s) {
-    const int g = run_map(A, B, in, out, nullptr, nullptr, nullptr, mask, dotv, partial, s);
+    const int g = run_map(A, B, in, EpiDot{dotv, out}, mask, partial, s);
     reduce_stage2<<<B, kThreads, 0, s>>>(g, B, partial, dot_out);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
@@ -1094,16 +1285,14 @@ int cg_loop_grid(int device) {
     std::lock_guard<std::mutex> lk(mu);
     auto it = grid.find(device);
     if (it != grid.end()) return it->second;
-    int sms = 0, coop = 0, occ1 = 0, occ2 = 0, occ4 = 0;
+    int sms = 0, coop = 0, occ = 0;
     int g = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, cg_loop_kernel<1>, kThreads, 0) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, cg_loop_kernel<2>, kThreads, 0) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ4, cg_loop_kernel<4>, kThreads, 0) == cudaSuccess) {
-        // three CTAs per SM (the launch bound of every form): the phases are
-        // latency-bound gathers that want the warps
-        const int per_sm = std::min(kLoopCtasPerSm, std::min(occ1, std::min(occ2, occ4)));
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cg_loop_kernel<kOdd, true, true>, kThreads, 0) == cudaSuccess) {
+        // three CTAs per SM (the launch bound): the phases are latency-bound
+        // gathers that want the warps
+        const int per_sm = std::min(kLoopCtasPerSm, occ);
         if (per_sm >= 1) g = sms * per_sm;
     }
     cudaGetLastError();
@@ -1118,14 +1307,10 @@ cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, int64_t nc,
                            unsigned int* bar, int* err, int* n_active, int* iters, int cap, int grid,
                            cudaStream_t s) {
     CgLoopArgs L;
-    // one instance per thread for a single instance (fewer registers); the
-    // unit layout is the 2-instance one, which has one chunk for B <= 2
-    const int ch = B == 1 ? 1 : (B <= 2 ? 2 : 4);
     L.A = A;
     L.AT = AT;
-    L.A.variant = L.AT.variant = (ch <= 2 ? 0 : 1);
-    L.blA = map_blocks(L.A, B);
-    L.blAT = map_blocks(L.AT, B);
+    L.blA = map_blocks(L.A, B, kThreads);
+    L.blAT = map_blocks(L.AT, B, kThreads);
     L.B = B;
     L.nc = nc;
     L.y = y;
@@ -1142,8 +1327,16 @@ cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, int64_t nc,
     L.iters = iters;
     L.cap = cap;
     void* args[] = {&L};
-    const void* fn = ch == 1 ? (const void*)cg_loop_kernel<1>
-                             : (ch == 2 ? (const void*)cg_loop_kernel<2> : (const void*)cg_loop_kernel<4>);
+    auto pick = [&](auto mode) -> const void* {
+        constexpr int MODE = decltype(mode)::value;
+        if (!A.packed || !AT.packed) return (const void*)cg_loop_kernel<MODE, false, false>;
+        return L.blA.deep && L.blAT.deep ? (const void*)cg_loop_kernel<MODE, true, true>
+                                         : (const void*)cg_loop_kernel<MODE, false, true>;
+    };
+    const LaneMode lm = lane_mode(B);
+    const void* fn = lm == kOne ? pick(std::integral_constant<int, kOne>())
+                                : (lm == kOdd ? pick(std::integral_constant<int, kOdd>())
+                                              : pick(std::integral_constant<int, kEven>()));
     const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, 0, s);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     return e;

@@ -97,20 +97,14 @@ struct DevBuf {
 // One map (A or A^T) on the device in the bucketed-ELL form of kernels.cuh.
 struct MapTable {
     DevBuf<int32_t> rows, cols, long_rows, long_ptr, long_col;
-    DevBuf<double> vals, long_val, book;
+    DevBuf<double> vals, long_val;
     DevMap dm;
 
     // Packs the coefficient of every ELL entry into its column word when the
     // columns fit in kCodeShift bits and the table has at most kBookSize
     // distinct coefficients (compared bit for bit, so the sums are unchanged);
     // returns the book, or an empty vector when the table stays unpacked.
-    // Only tables larger than L2 are packed: there the coefficient stream is
-    // HBM traffic (H50: 10 % faster maps), while for tables that stay in L2
-    // the book lookup costs more than it saves (H10 and 19 x n = 20: 2-3 %
-    // slower on B200).
-    static constexpr size_t kPackMinBytes = size_t(128) << 20;
     static std::vector<double> pack(std::vector<int32_t>& hcols, const std::vector<double>& hvals) {
-        if (hcols.size() * (sizeof(int32_t) + sizeof(double)) < kPackMinBytes) return {};
         std::map<uint64_t, int> code;
         std::vector<double> bk;
         for (size_t k = 0; k < hcols.size(); k++) {
@@ -135,7 +129,7 @@ struct MapTable {
     }
 
     void build(const Csr& M) {
-        static const int widths[kMaxBuckets] = {1, 2, 4, 8, 16, 32};
+        static const int widths[kMaxBuckets] = {1, 2, 4, 5, 8, 16, 32};
         std::vector<std::vector<int32_t>> brow(kMaxBuckets);
         std::vector<int32_t> lrows, lptr(1, 0), lcol;
         std::vector<double> lval;
@@ -147,12 +141,24 @@ struct MapTable {
                 brow[w].push_back((int32_t)r);
             } else {
                 lrows.push_back((int32_t)r);
-                for (int64_t k = M.rowptr[r]; k < M.rowptr[r + 1]; k++) {
-                    lcol.push_back(M.col[k]);
-                    lval.push_back(M.val[k]);
-                }
-                lptr.push_back((int32_t)lcol.size());
             }
+        }
+        // The rows a warp takes first, then those of a whole CTA.  A warp sums
+        // a row of 200 entries for 20 instances in 50 us, alone at the end of
+        // the launch: that pays only where there are many such rows (the
+        // contractions of A^T), not for the handful of trace rows.
+        std::map<int64_t, int> same;
+        for (int32_t r : lrows) same[M.rowptr[r + 1] - M.rowptr[r]]++;
+        const auto mid_end = std::stable_partition(lrows.begin(), lrows.end(), [&](int32_t r) {
+            const int64_t len = M.rowptr[r + 1] - M.rowptr[r];
+            return len <= kMidRow && same[len] >= kMidMany;
+        });
+        for (int32_t r : lrows) {
+            for (int64_t k = M.rowptr[r]; k < M.rowptr[r + 1]; k++) {
+                lcol.push_back(M.col[k]);
+                lval.push_back(M.val[k]);
+            }
+            lptr.push_back((int32_t)lcol.size());
         }
         // inside a bucket, rows are ordered by their first column: rows that
         // gather from the same region of the input run in the same CTA wave,
@@ -192,10 +198,7 @@ struct MapTable {
         const std::vector<double> bk = pack(hcols, hvals);
         rows.upload(hrows.data(), hrows.size());
         cols.upload(hcols.data(), hcols.size());
-        if (bk.empty())
-            vals.upload(hvals.data(), hvals.size());
-        else
-            book.upload(bk.data(), bk.size());
+        if (bk.empty()) vals.upload(hvals.data(), hvals.size());
         long_rows.upload(lrows.data(), lrows.size());
         long_ptr.upload(lptr.data(), lptr.size());
         long_col.upload(lcol.data(), lcol.size());
@@ -203,8 +206,10 @@ struct MapTable {
         dm.rows = rows.p;
         dm.cols = cols.p;
         dm.vals = bk.empty() ? vals.p : nullptr;
-        dm.book = bk.empty() ? nullptr : book.p;
+        dm.packed = !bk.empty();
+        std::copy(bk.begin(), bk.end(), dm.book);
         dm.nlong = (int)lrows.size();
+        dm.nmid = (int)(mid_end - lrows.begin());
         dm.long_rows = long_rows.p;
         dm.long_ptr = long_ptr.p;
         dm.long_col = long_col.p;
