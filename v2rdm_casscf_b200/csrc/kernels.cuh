@@ -26,6 +26,10 @@ extern std::atomic<long> g_kernel_launches;
 // each, the others by a whole CTA.
 constexpr int kMaxBuckets = 7;
 constexpr int kMidRow = 256, kMidMany = 32;
+constexpr int kLongClasses = 5;  // rows of up to 16, 32, 64, 128 and 256 entries
+// maps with fewer rows are bound by latency at small batches: their rows of 17
+// to 32 entries take a warp each too, instead of one thread
+constexpr int kLatencyRows = 1 << 18;
 constexpr int kCodeShift = 27;                 // packed entry: 27 column bits, 4 code bits
 constexpr int kBookSize = 1 << (31 - kCodeShift);  // 16 coefficients at most
 struct DevMap {
@@ -50,6 +54,14 @@ struct DevMap {
     const int32_t* long_ptr = nullptr;
     const int32_t* long_col = nullptr;
     const double* long_val = nullptr;
+    // the same rows sorted by length with packed entries, for the resident CG
+    // (a packed table with no row above 256 entries; else nres = -1), and the
+    // end of each length class among them
+    int nres = -1;
+    int res_upto[kLongClasses] = {};
+    const int32_t* res_row = nullptr;
+    const int32_t* res_ptr = nullptr;
+    const int32_t* res_word = nullptr;
     // kernel variant chosen by the autotuner for one instance count (-1: the
     // built-in rule); see kMapVariants
     int variant = -1;
@@ -62,10 +74,6 @@ constexpr int kMapVariants = 2;  // 0: plain, 1: streamed
 // (each of sub, coef, add optional); instances with mask[b] == 0 are skipped.
 void launch_spmv(const DevMap& A, int B, const double* in, double* out, const double* sub, const double* coef,
                  const double* add, const int* mask, cudaStream_t s);
-
-// out = A in, and dot_out[b] = sum_r dotv[r,b] out[r,b] (deterministic).
-void launch_spmv_dot(const DevMap& A, int B, const double* in, double* out, const double* dotv, const int* mask,
-                     double* partial, double* dot_out, cudaStream_t s);
 
 // Per-instance reductions over interleaved vectors of n elements.
 enum ReduceMode {
@@ -91,7 +99,7 @@ struct CgScalars {
     double rrmin;  // smallest r.r of this solve
     int active;    // still iterating
     int iter;      // iter_ of the reference
-    int do_p;      // p update pending this iteration
+    int step;      // this iteration takes a step (q.q above rounding noise)
     int maxiter;
     int stalled;   // stopped because r.r grew past kCgGrowth * rrmin
 };
@@ -103,51 +111,48 @@ struct CgScalars {
 // in 4,252 CG solves); a rise past this factor stops the instance's CG with
 // the current y instead.
 constexpr double kCgGrowth = 1e4;
-// r = rhs - Ap ; p = r
-void launch_cg_init(int64_t n, int B, const double* rhs, const double* Ap, double* r, double* p, const CgScalars* cs,
-                    cudaStream_t s);
-// alpha = rr / pap
-void launch_cg_alpha(int B, CgScalars* cs, const double* pap, cudaStream_t s);
-// y += alpha p ; r -= alpha Ap ; rr_out[b] = r.r
-void launch_cg_update_yr(int64_t n, int B, double* y, double* r, const double* p, const double* Ap,
-                         const CgScalars* cs, double* partial, double* rr_out, cudaStream_t s);
-// convergence test and beta; counts instances still active into *n_active
-void launch_cg_beta(int B, CgScalars* cs, const double* rrnew, int* n_active, cudaStream_t s);
-// One CG step after p.Ap (in pap): y += alpha p, r -= alpha Ap, then r.r,
-// alpha, the convergence test, beta and the count of instances still
-// iterating into *n_active (two launches; replaces alpha / update_yr / beta)
-void launch_cg_step(int64_t n, int B, double* y, double* r, const double* p, const double* Ap, CgScalars* cs,
-                    const double* pap, double* partial, int* n_active, cudaStream_t s);
-// p = beta p + r
-void launch_cg_update_p(int64_t n, int B, double* p, const double* r, const CgScalars* cs, cudaStream_t s);
+// The CG of a group as map applications with the vector updates in their
+// epilogues (maps.cu, EpiCgQ): r = rhs - A q for q = A^T y and its r.r; then
+// per iteration the direction q = A^T r + beta q with alpha from q.q, and the
+// step p = r + beta p, y += alpha p, r -= alpha A q with the convergence test
+// and beta from r.r, counting the instances still iterating into *n_active.
+// Instances with cs[b].active == 0 are left alone.  partial holds
+// reduce_partial_size(B) doubles.
+void launch_cg_start(const DevMap& A, int B, const double* q, const double* rhs, double* r, CgScalars* cs,
+                     double* partial, int* n_active, cudaStream_t s);
+void launch_cg_direction(const DevMap& AT, int B, const double* r, double* q, CgScalars* cs, double* partial,
+                         int* n_active, cudaStream_t s);
+void launch_cg_step(const DevMap& A, int B, const double* q, double* y, double* r, double* p, CgScalars* cs,
+                    double* partial, int* n_active, cudaStream_t s);
 // Sets the WHILE condition h of a device-side CG loop: ++*count, then
 // continue while *n_active > 0 and *count < cap.
 void launch_cg_while(cudaGraphConditionalHandle h, const int* n_active, int* count, int cap, cudaStream_t s);
 
 // Persistent CG (maps.cu): a whole CG solve of a small group in one
-// cooperative launch.  Groups of at most kLoopMaxB instances and
-// kLoopMaxElems constraint elements (nc * B), where launch latency, not
-// bandwidth, bounds an iteration.
+// cooperative launch.  Groups of at most kLoopMaxB instances and kLoopMaxRows
+// constraints (n <= 13 with DQG), where launch latency, not bandwidth, bounds
+// an iteration; above, two map launches with their reductions are faster
+// (B200, us per iteration, persistent / launches: n = 12 one instance 25.6 /
+// 29.7, n = 10 eight instances 41.5 / 46.5, n = 14 one instance 43.2 / 39.6,
+// n = 20 one instance 131 / 99).
 constexpr int kLoopMaxB = 8;
-constexpr int64_t kLoopMaxElems = 1 << 21;
+constexpr int64_t kLoopMaxRows = 300000;
 bool cg_loop_fits(int64_t nc, int B);
 // CTAs of the cooperative grid on this device (0: no cooperative launch)
 int cg_loop_grid(int device);
-// Iterates until no instance of cs is active or cap iterations: y, r, p and
-// cs as the chunked path leaves them; *n_active the instances still active,
-// *iters the iterations run, *err = 1 if a grid barrier wait ran out (then the
-// results are invalid).  *bar must be 0 at the launch.  part_dot holds
-// (row tiles + long rows of A) x B, part_rr grid x B doubles.
-cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, int64_t nc, double* y, double* r, double* p,
-                           double* atp, double* ap, CgScalars* cs, double* part_dot, double* part_rr,
-                           unsigned int* bar, int* err, int* n_active, int* iters, int cap, int grid,
-                           cudaStream_t s);
+size_t cg_loop_slots(int grid, int B);
+// The whole solve from y, rhs and cs (tol, active, maxiter set): iterates
+// until no instance is active or cap iterations; y, r, p, q and cs as the
+// launches above leave them; *n_active the instances still active, *iters the
+// iterations run, *err = 1 if a wait of the grid's exchanges ran out
+// (then the results are invalid; *err must be 0 at the launch).  slots holds
+// cg_loop_slots(grid, B) words.
+cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, const double* rhs, double* y, double* r, double* p,
+                           double* q, CgScalars* cs, unsigned long long* slots, int* err, int* n_active,
+                           int* iters, int cap, int grid, cudaStream_t s);
 // CG start extrapolation over [e * B + b]: where mode[b] == 2,
 // y <- y + (y - yprev); where mode[b] >= 1, yprev <- y (its value on entry)
 void launch_cg_extrapolate(int64_t n, int B, double* y, double* yprev, const int* mode, cudaStream_t s);
-// rr <- initial r.r
-void launch_cg_set_rr(int B, CgScalars* cs, const double* rr, int* n_active, cudaStream_t s);
-
 // ---- Anderson acceleration of the outer iteration --------------------------
 // The state w = (x, z) of one instance is the 2 * nx rows e < nx of x and
 // e >= nx of z, interleaved [e * B + b] like every vector; the history holds

@@ -65,7 +65,7 @@ __device__ __forceinline__ Chunk chunk_of(int64_t nrows, int B) {
 // thread b walks its rows.  The CTA synchronises on entry and on exit, so
 // the shared scratch can be reused right away.
 __device__ __forceinline__ double cta_instance_sum(double v, int B) {
-    __shared__ double sh[kThreads];
+    __shared__ double sh[1024];  // the largest CTA
     double s = 0.0;
     __syncthreads();
     if ((32 % B) == 0) {
@@ -87,13 +87,6 @@ __device__ __forceinline__ double cta_instance_sum(double v, int B) {
     return s;
 }
 
-// Per-instance block partial of v, written to partial[slot * B + b] (slot is
-// the block's index among the partial sums, not always blockIdx.x).
-__device__ __forceinline__ void block_partial(double v, int B, double* __restrict__ partial, int64_t slot) {
-    const double s = cta_instance_sum(v, B);
-    if ((int)threadIdx.x < B) partial[slot * B + threadIdx.x] = s;
-}
-
 // ---- the map kernels ---------------------------------------------------------
 //
 // Lanes run along the instances of a row: each of its lanes_of(B) lanes serves
@@ -113,7 +106,8 @@ __device__ __forceinline__ void block_partial(double v, int B, double* __restric
 //   n = 28, 1 instance     243 ->  83 us
 //   n = 8 T2, 3 instances   99 ->  37 us
 //   n = 10, 1 instance     11.6 -> 9.8 us
-constexpr int kWarps = kThreads / 32;
+constexpr int kLoopThreads = 512;  // CTA of the persistent CG
+constexpr int kWarps = 32;         // of the largest CTA
 
 // How instances map to lanes: one lane each (B = 1), or two instances per
 // lane: l and l + (B + 1) / 2 for odd B (contiguous 8-byte loads), 2 l and
@@ -121,6 +115,21 @@ constexpr int kWarps = kThreads / 32;
 enum LaneMode { kOne = 0, kOdd = 1, kEven = 2 };
 __host__ __device__ constexpr int lanes_of(int B) { return (B + 1) / 2; }
 static LaneMode lane_mode(int B) { return B == 1 ? kOne : ((B & 1) ? kOdd : kEven); }
+
+// Sum of v over the CTA, to thread 0: one synchronisation.  The scratch is free
+// again after the CTA's next one.
+__device__ __forceinline__ double cta_sum(double v) {
+    __shared__ double sh[kWarps];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x < 32) {
+        if (threadIdx.x < (blockDim.x >> 5)) s = sh[threadIdx.x];
+        for (int o = kWarps / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    }
+    return threadIdx.x == 0 ? s : 0.0;
+}
 
 // Work units of one map application: first the long rows (a CTA each), then
 // the mid rows (a warp each, 32 instances at a time), then the row tiles.
@@ -132,6 +141,11 @@ struct Blocks {
     int deep;                    // the deep form: ell_depth(width) rows per thread
 };
 
+// Slots whose gathers a thread issues together in rows of eight and more: all
+// of them where latency counts, four in the deep form (registers: the batch of
+// eight made A^T at n = 20 with 19 instances 213 us instead of 151).
+__host__ __device__ constexpr int wide_batch(bool deep) { return deep ? 4 : 8; }
+
 // Rows per thread of the deep form, by bucket width.
 __host__ __device__ constexpr int ell_depth(int W) { return W == 1 ? 4 : (W == 2 ? 2 : 1); }
 
@@ -142,17 +156,17 @@ struct Lane {
     bool on0, on1;   // instances present and not masked
 };
 
-template <int MODE>
-__device__ __forceinline__ Lane lane_of(int B, const int* mask) {
+template <int MODE, class Epi>
+__device__ __forceinline__ Lane lane_of(int B, const Epi& e) {
     Lane L;
-    const int n = lanes_of(B), l = (int)threadIdx.x % n;
-    L.B = B;
+    const int n = MODE == kOne ? 1 : lanes_of(B), l = MODE == kOne ? 0 : (int)threadIdx.x % n;
+    L.B = MODE == kOne ? 1 : B;
     L.rpp = (int)blockDim.x / n;
     L.rsub = (int)threadIdx.x / n;
     L.b0 = MODE == kEven ? 2 * l : l;
     L.b1 = MODE == kEven ? 2 * l + 1 : (MODE == kOdd ? l + n : B);
-    L.on0 = !mask || mask[L.b0];
-    L.on1 = MODE != kOne && L.b1 < B && (!mask || mask[L.b1]);
+    L.on0 = e.on(L.b0);
+    L.on1 = MODE != kOne && L.b1 < B && e.on(L.b1);
     return L;
 }
 
@@ -208,15 +222,24 @@ __device__ __forceinline__ double2 load_two(const double* p, bool ok) {
     return v;
 }
 
-// What happens to the sum s of row r for instance b.  The returned values are
-// summed per instance where kSum is set.
+// What happens to the sum s of row r for instance b: own() loads what the row
+// itself needs (issued beside the gathers where a thread has one row), one()
+// finishes it; one()'s values are summed per instance where kSum is set.
+struct OwnNone {};
 
-// out = A in
+// out = A in, for the instances of mask (null: all)
 struct EpiStore {
     static constexpr bool kSum = false;
     double* out;
+    const int* mask;
+    __device__ __forceinline__ bool on(int b) const { return !mask || mask[b]; }
+    using Own = OwnNone;
     template <bool COH>
-    __device__ __forceinline__ double one(int32_t r, int B, int b, double s) const {
+    __device__ __forceinline__ Own own(int32_t, int, int) const {
+        return {};
+    }
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t r, int B, int b, double s, const Own&) const {
         out[(int64_t)r * B + b] = s;
         return 0.0;
     }
@@ -228,8 +251,15 @@ struct EpiAffine {
     const double* coef;
     const double* add;
     double* out;
+    const int* mask;
+    __device__ __forceinline__ bool on(int b) const { return !mask || mask[b]; }
+    using Own = OwnNone;
     template <bool COH>
-    __device__ __forceinline__ double one(int32_t r, int B, int b, double s) const {
+    __device__ __forceinline__ Own own(int32_t, int, int) const {
+        return {};
+    }
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t r, int B, int b, double s, const Own&) const {
         const int64_t t = (int64_t)r * B + b;
         if (sub) s -= sub[r];
         if (coef) s *= coef[b];
@@ -238,21 +268,92 @@ struct EpiAffine {
         return 0.0;
     }
 };
-// out = A in, summing dotv . out
-struct EpiDot {
+
+// The CG iteration (cg_solver.cc:141-177) in two map applications, every
+// vector update in the epilogue of the map that produces its input:
+//   q = A^T r + beta q   (= A^T p for the new p = r + beta p), summing q.q = p.A A^T p
+//   p = r + beta p, y += alpha p, r -= alpha A q, summing r.r
+// The textbook order (A^T p, A (A^T p) with p.Ap, then y and r, then p) has
+// four passes with a reduction or a barrier after each and moves 12 vectors of
+// constraint length and 2 of primal length per iteration; this one has two
+// passes and moves 7 and 3 (B200, us per CG iteration: 19 instances of n = 17
+// 716 -> 443, 12 of n = 14 227 -> 164, one of n = 20 161 -> 100).  Elements of r, p, y and q other than r's and q's
+// gathers are touched only by the thread that owns the row.
+struct EpiCgQ {
     static constexpr bool kSum = true;
-    const double* dotv;
-    double* out;
+    const CgScalars* cs;
+    double* q;
+    struct Own {
+        double q;
+    };
+    __device__ __forceinline__ bool on(int b) const { return cs[b].active; }
     template <bool COH>
-    __device__ __forceinline__ double one(int32_t r, int B, int b, double s) const {
-        const int64_t t = (int64_t)r * B + b;
-        out[t] = s;
-        return (COH ? __ldcg(dotv + t) : dotv[t]) * s;
+    __device__ __forceinline__ Own own(int32_t r, int B, int b) const {
+        const double* p = q + (int64_t)r * B + b;
+        // beta = 0 in the first iteration, where q holds an earlier solve's values
+        return {cs[b].beta != 0.0 ? (COH ? __ldcg(p) : *p) : 0.0};
+    }
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t r, int B, int b, double s, const Own& o) const {
+        s += cs[b].beta * o.q;
+        q[(int64_t)r * B + b] = s;
+        return s * s;
+    }
+};
+struct EpiCgR {
+    static constexpr bool kSum = true;
+    const CgScalars* cs;
+    double *y, *r, *p;
+    struct Own {
+        double y, r, p;
+    };
+    __device__ __forceinline__ bool on(int b) const { return cs[b].step; }
+    template <bool COH>
+    __device__ __forceinline__ Own own(int32_t row, int B, int b) const {
+        const int64_t t = (int64_t)row * B + b;
+        Own o;
+        o.y = COH ? __ldcg(y + t) : y[t];
+        o.r = COH ? __ldcg(r + t) : r[t];
+        o.p = 0.0;
+        if (cs[b].beta != 0.0) o.p = COH ? __ldcg(p + t) : p[t];
+        return o;
+    }
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t row, int B, int b, double s, const Own& o) const {
+        const int64_t t = (int64_t)row * B + b;
+        const double alpha = cs[b].alpha;
+        const double pv = o.r + cs[b].beta * o.p;
+        p[t] = pv;
+        y[t] = o.y + alpha * pv;
+        const double rv = o.r - alpha * s;
+        r[t] = rv;
+        return rv * rv;
+    }
+};
+// r = rhs - A (A^T y), summing r.r
+struct EpiCgInit {
+    static constexpr bool kSum = true;
+    const CgScalars* cs;
+    const double* rhs;
+    double* r;
+    struct Own {
+        double rhs;
+    };
+    __device__ __forceinline__ bool on(int b) const { return cs[b].active; }
+    template <bool COH>
+    __device__ __forceinline__ Own own(int32_t row, int B, int b) const {
+        return {rhs[(int64_t)row * B + b]};
+    }
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t row, int B, int b, double s, const Own& o) const {
+        const double rv = o.rhs - s;
+        r[(int64_t)row * B + b] = rv;
+        return rv * rv;
     }
 };
 
-// The tiles t0, t0 + tstep, ... of bucket bi, whose width is 1, 2, 5 (WB) or a
-// multiple of four (WB = 4, nbatch batches of slots).  A bucket has fewer than
+// The tiles t0, t0 + tstep, ... of bucket bi, whose width is 1, 2, 4, 5 (WB) or
+// a multiple of eight (nbatch batches of wide_batch slots).  A bucket has fewer than
 // 2^32 table entries (the table has fewer than 2^31, and padding at most
 // doubles a row), so table offsets are 32-bit.
 template <int WB, int MODE, bool DEEP, bool STREAM, bool PK, bool COH, class Epi>
@@ -260,6 +361,7 @@ __device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int nbatch, in
                                          const double* __restrict__ in, const Epi& e, const double* sbook,
                                          double (&dot)[2]) {
     constexpr int R = DEEP ? ell_depth(WB) : 1;
+    constexpr bool WIDE = WB == wide_batch(DEEP);  // also the bucket of four in the deep form, with one batch
     constexpr int32_t kCol = PK ? (1 << kCodeShift) - 1 : -1;
     static_assert(!DEEP || PK, "the deep form reads packed tables");
     const uint32_t ns = (uint32_t)M.nslots[bi];
@@ -292,10 +394,15 @@ __device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int nbatch, in
         const bool more = next < ns;
         double a0[R], a1[R];
         int32_t rn[R];
+        typename Epi::Own o0[R], o1[R];
 #pragma unroll
         for (int j = 0; j < R; j++) a0[j] = a1[j] = 0.0;
+        if (!DEEP) {
+            if (L.on0) o0[0] = e.template own<COH>(r[0], L.B, L.b0);
+            if (MODE != kOne && L.on1) o1[0] = e.template own<COH>(r[0], L.B, L.b1);
+        }
 #pragma unroll 1
-        for (int kb = 0; kb < (WB == 4 ? nbatch : 1); kb++) {
+        for (int kb = 0; kb < (WIDE ? nbatch : 1); kb++) {
             double g0[WB][R], g1[WB][R], v[WB][R];
 #pragma unroll
             for (int k = 0; k < WB; k++)
@@ -318,7 +425,7 @@ __device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int nbatch, in
                         v[k][j] = load_one<false>(vals + (size_t)((kb * WB + k) * ns + (uint32_t)i + j * rpp), ok);
                 }
             int32_t wn[WB][R];
-            if (WB == 4 && kb + 1 < nbatch) {
+            if (WIDE && kb + 1 < nbatch) {
                 load((uint32_t)i, (kb + 1) * WB, true, wn);  // the next batch of slots
             } else if (DEEP) {
                 load((uint32_t)next, 0, more, wn);  // the next tile's first
@@ -332,14 +439,16 @@ __device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int nbatch, in
                     const double c = PK ? sbook[(w[k][j] >> kCodeShift) & (kBookSize - 1)] : v[k][j];
                     a0[j] += c * g0[k][j];
                     if (MODE != kOne) a1[j] += c * g1[k][j];
-                    if (DEEP || WB == 4) w[k][j] = wn[k][j];
+                    if (DEEP || WIDE) w[k][j] = wn[k][j];
                 }
         }
 #pragma unroll
         for (int j = 0; j < R; j++) {
             if (r[j] >= 0) {
-                if (L.on0) dot[0] += e.template one<COH>(r[j], L.B, L.b0, a0[j]);
-                if (MODE != kOne && L.on1) dot[1] += e.template one<COH>(r[j], L.B, L.b1, a1[j]);
+                if (DEEP && L.on0) o0[j] = e.template own<COH>(r[j], L.B, L.b0);
+                if (DEEP && MODE != kOne && L.on1) o1[j] = e.template own<COH>(r[j], L.B, L.b1);
+                if (L.on0) dot[0] += e.template one<COH>(r[j], L.B, L.b0, a0[j], o0[j]);
+                if (MODE != kOne && L.on1) dot[1] += e.template one<COH>(r[j], L.B, L.b1, a1[j], o1[j]);
             }
             if (DEEP) r[j] = rn[j];
         }
@@ -373,7 +482,7 @@ __device__ __forceinline__ double warps_to_instances(double v, int c0, int cnt) 
 // entries on 256 threads each (38 us of a 48 us launch at one instance).
 template <bool COH, class Epi>
 __device__ __forceinline__ double mid_rows(const DevMap& M, int B, const double* __restrict__ in, const Epi& e,
-                                           const int* __restrict__ mask, int group, int chunk) {
+                                           int group, int chunk) {
     const int lane = threadIdx.x & 31;
     const int m = group * (int)(blockDim.x >> 5) + (threadIdx.x >> 5);
     const int c0 = chunk * 32, cnt = B - c0 < 32 ? B - c0 : 32;
@@ -395,7 +504,10 @@ __device__ __forceinline__ double mid_rows(const DevMap& M, int B, const double*
             if (l < left - h) s += o;
             left = h;
         }
-        if (lane < cnt && !(mask && !mask[b])) res = e.template one<COH>(M.long_rows[m], B, b, s);
+        if (lane < cnt && e.on(b)) {
+            const int32_t r = M.long_rows[m];
+            res = e.template one<COH>(r, B, b, s, e.template own<COH>(r, B, b));
+        }
     }
     return res;
 }
@@ -404,7 +516,7 @@ __device__ __forceinline__ double mid_rows(const DevMap& M, int B, const double*
 // ... for instance t % B, then a fixed-order reduction per instance.
 template <bool COH, class Epi>
 __device__ __forceinline__ double long_row(const DevMap& M, int B, const double* __restrict__ in, const Epi& e,
-                                           const int* __restrict__ mask, int lr) {
+                                           int lr) {
     const int lanes = blockDim.x / B;
     const int b = threadIdx.x % B;
     const int l = threadIdx.x / B;
@@ -419,8 +531,10 @@ __device__ __forceinline__ double long_row(const DevMap& M, int B, const double*
     }
     const double t = cta_instance_sum(s, B);
     double acc = 0.0;
-    if ((int)threadIdx.x < B && !(mask && !mask[threadIdx.x]))
-        acc = e.template one<COH>(M.long_rows[lr], B, (int)threadIdx.x, t);
+    if ((int)threadIdx.x < B && e.on(threadIdx.x)) {
+        const int32_t r = M.long_rows[lr];
+        acc = e.template one<COH>(r, B, (int)threadIdx.x, t, e.template own<COH>(r, B, (int)threadIdx.x));
+    }
     return acc;
 }
 
@@ -428,27 +542,30 @@ __device__ __forceinline__ double long_row(const DevMap& M, int B, const double*
 // optional dot for instance b (fixed order; 0 elsewhere).
 template <int MODE, bool DEEP, bool STREAM, bool PK, bool COH, class Epi>
 __device__ __forceinline__ double ell_cta(const DevMap& M, const Blocks& bl, int B, const double* __restrict__ in,
-                                          const Epi& e, const int* mask, const double* sbook) {
+                                          const Epi& e, const double* sbook) {
     const int G = (int)gridDim.x;
     double sum = 0.0;  // thread b: instance b
     int u = (int)blockIdx.x;
     for (; u < bl.mid; u += G) {
-        const double d = long_row<COH>(M, B, in, e, mask, M.nmid + u);
+        const double d = long_row<COH>(M, B, in, e, M.nmid + u);
         if (Epi::kSum) sum += d;
     }
     for (; u < bl.start[0]; u += G) {
         const int chunk = (u - bl.mid) % bl.midchunks, c0 = chunk * 32;
-        const double d = mid_rows<COH>(M, B, in, e, mask, (u - bl.mid) / bl.midchunks, chunk);
+        const double d = mid_rows<COH>(M, B, in, e, (u - bl.mid) / bl.midchunks, chunk);
         if (Epi::kSum) sum += warps_to_instances(d, c0, B - c0 < 32 ? B - c0 : 32);
     }
-    const Lane L = lane_of<MODE>(B, mask);
+    const Lane L = lane_of<MODE>(B, e);
     double dot[2] = {0.0, 0.0};
     if (L.rsub < L.rpp && (L.on0 || L.on1)) {
 #pragma unroll 1
         for (int bi = 0; bi < M.nb; bi++) {
             // the first unit of this bucket that is this CTA's
-            int t0 = ((int)blockIdx.x - bl.start[bi]) % G;
-            if (t0 < 0) t0 += G;
+            int t0 = (int)blockIdx.x - bl.start[bi];
+            if (t0 < 0) {
+                if (G >= bl.start[kMaxBuckets]) break;  // one unit per CTA
+                t0 = (t0 % G + G) % G;
+            }
             if (t0 >= bl.start[bi + 1] - bl.start[bi]) continue;
             const int W = M.width[bi];
             if (W == 1)
@@ -457,18 +574,21 @@ __device__ __forceinline__ double ell_cta(const DevMap& M, const Blocks& bl, int
                 ell_rows<2, MODE, DEEP, STREAM, PK, COH>(M, bi, 1, t0, G, L, in, e, sbook, dot);
             else if (W == 5)
                 ell_rows<5, MODE, DEEP, STREAM, PK, COH>(M, bi, 1, t0, G, L, in, e, sbook, dot);
+            else if (W == 4)
+                ell_rows<4, MODE, DEEP, STREAM, PK, COH>(M, bi, 1, t0, G, L, in, e, sbook, dot);
             else
-                ell_rows<4, MODE, DEEP, STREAM, PK, COH>(M, bi, W / 4, t0, G, L, in, e, sbook, dot);
+                ell_rows<wide_batch(DEEP), MODE, DEEP, STREAM, PK, COH>(M, bi, W / wide_batch(DEEP), t0, G, L, in, e,
+                                                                        sbook, dot);
         }
     }
     if (Epi::kSum) {
-        // two instances per lane: fold each half on its own, then to thread b
-        const int n = lanes_of(B);
-        const double s0 = cta_instance_sum(dot[0], n);
         if (MODE == kOne) {
-            sum += s0;
+            sum += cta_sum(dot[0]);
         } else {
-            __shared__ double sh[kThreads];
+            // two instances per lane: fold each half on its own, then to thread b
+            const int n = lanes_of(B);
+            const double s0 = cta_instance_sum(dot[0], n);
+            __shared__ double sh[256];  // one per instance
             const double s1 = cta_instance_sum(dot[1], n);
             if ((int)threadIdx.x < n) {
                 sh[MODE == kEven ? 2 * threadIdx.x : threadIdx.x] = s0;
@@ -486,15 +606,14 @@ __device__ __forceinline__ double ell_cta(const DevMap& M, const Blocks& bl, int
 template <int MODE, bool DEEP, bool STREAM, bool PK, class Epi>
 __global__ void __launch_bounds__(kThreads, kMapCtasPerSm)
     ell_kernel(const __grid_constant__ DevMap M, const __grid_constant__ Blocks bl, int B,
-               const double* __restrict__ in, const __grid_constant__ Epi e, const int* __restrict__ mask,
-               double* __restrict__ partial) {
+               const double* __restrict__ in, const __grid_constant__ Epi e, double* __restrict__ partial) {
     // the coefficient book of a packed table, in shared memory
     __shared__ double sbook[kBookSize];
     if (PK) {
         if (threadIdx.x < kBookSize) sbook[threadIdx.x] = M.book[threadIdx.x];
         __syncthreads();
     }
-    const double s = ell_cta<MODE, DEEP, STREAM, PK, false>(M, bl, B, in, e, mask, sbook);
+    const double s = ell_cta<MODE, DEEP, STREAM, PK, false>(M, bl, B, in, e, sbook);
     if (Epi::kSum && (int)threadIdx.x < B) partial[(int64_t)blockIdx.x * B + threadIdx.x] = s;
 }
 
@@ -698,116 +817,25 @@ __global__ void aa_mix_kernel(int64_t nx, int B, int m, double* __restrict__ x, 
     }
 }
 
-__global__ void cg_init_kernel(int64_t n, int B, const double* __restrict__ rhs, const double* __restrict__ Ap,
-                               double* __restrict__ r, double* __restrict__ p, const CgScalars* __restrict__ cs) {
-    const int64_t total = n * B;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int b = (int)(t % B);
-        if (!cs[b].active) continue;
-        const double v = rhs[t] - Ap[t];
-        r[t] = v;
-        p[t] = v;
-    }
+// The scalars of cg_solver.cc:141-177.  After q.q: alpha, unless q is zero or
+// rounding noise next to r (p then has no component outside the null space of
+// A^T; |p| >= |r|, and the smallest nonzero eigenvalue of A A^T is of order
+// 0.1, so a ratio below 1e-26 cannot be anything else): no step.
+constexpr double kCgNull = 1e-26;
+__device__ __forceinline__ void cg_scalar_alpha(CgScalars& c, double qq) {
+    c.pap = qq;
+    c.step = c.active && qq > kCgNull * c.rr;
+    c.alpha = c.step ? c.rr / qq : 0.0;
 }
-
-__global__ void cg_set_rr_kernel(int B, CgScalars* cs, const double* rr, int* n_active) {
-    int cnt = 0;
-    for (int b = threadIdx.x; b < B; b += blockDim.x) {
-        if (cs[b].active) {
-            cs[b].rr = rr[b];
-            cs[b].rrmin = rr[b];
-            cnt++;
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    if (threadIdx.x == 0) *n_active = cnt;
-}
-
-__global__ void cg_alpha_kernel(int B, CgScalars* cs, const double* pap) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B || !cs[b].active) return;
-    cs[b].pap = pap[b];
-    if (!(pap[b] > 0.0)) {
-        // p has no component outside the null space of A^T (or r = 0): no step
-        cs[b].alpha = 0.0;
-        cs[b].active = 0;
-        cs[b].stalled = 1;
-        return;
-    }
-    cs[b].alpha = cs[b].rr / pap[b];
-}
-
-// y += alpha p ; r -= alpha Ap ; partial[., b] of r.r (cg_solver.cc:159-165)
-__global__ void cg_update_yr_kernel(int64_t n, int B, double* __restrict__ y, double* __restrict__ r,
-                                    const double* __restrict__ p, const double* __restrict__ Ap,
-                                    const CgScalars* __restrict__ cs, double* __restrict__ partial) {
-    const Chunk ch = chunk_of(n, B);
-    double acc = 0.0;
-    if (ch.live) {
-        const int b = ch.b;
-        const bool act = cs[b].active;
-        const double a = cs[b].alpha;
-        for (int64_t e = ch.first; e < ch.nrows; e += ch.stride) {
-            const int64_t t = e * B + b;
-            double rv = r[t];
-            if (act) {
-                y[t] += a * p[t];
-                rv += -a * Ap[t];
-                r[t] = rv;
-            }
-            acc += rv * rv;
-        }
-    }
-    block_partial(acc, B, partial, blockIdx.x);
-}
-
-// y += alpha p ; r -= alpha Ap with alpha = r.r / p.Ap computed by every
-// thread from the instance's scalars (no separate alpha launch; p.Ap <= 0
-// takes no step and the beta kernel stops the instance); partial[., b] of
-// r.r.  Block 0 clears the active-instance counter that the beta kernel
-// fills.
-__global__ void cg_step_yr_kernel(int64_t n, int B, double* __restrict__ y, double* __restrict__ r,
-                                  const double* __restrict__ p, const double* __restrict__ Ap,
-                                  const CgScalars* __restrict__ cs, const double* __restrict__ pap,
-                                  double* __restrict__ partial, int* __restrict__ n_active) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *n_active = 0;
-    const Chunk ch = chunk_of(n, B);
-    double acc = 0.0;
-    if (ch.live) {
-        const int b = ch.b;
-        const double pp = pap[b];
-        const bool act = cs[b].active && pp > 0.0;
-        const double a = act ? cs[b].rr / pp : 0.0;
-        for (int64_t e = ch.first; e < ch.nrows; e += ch.stride) {
-            const int64_t t = e * B + b;
-            double rv = r[t];
-            if (act) {
-                y[t] += a * p[t];
-                rv += -a * Ap[t];
-                r[t] = rv;
-            }
-            acc += rv * rv;
-        }
-    }
-    block_partial(acc, B, partial, blockIdx.x);
-}
-
-// The scalars of cg_solver.cc:159-177 after a step with p.Ap = pap and the new
-// r.r = rn: alpha, the ||r|| < tol test, beta and the iteration count, the
-// stops on p.Ap <= 0 and on residual growth (kCgGrowth).
-__device__ __forceinline__ void cg_scalar_step(CgScalars& c, double pap, double rn) {
-    c.do_p = 0;
+// After r.r = rn: the ||r|| < tol test, beta and the iteration count, the stop
+// without a step and the stop on residual growth (kCgGrowth).
+__device__ __forceinline__ void cg_scalar_beta(CgScalars& c, double rn) {
     if (!c.active) return;
-    c.pap = pap;
-    if (!(c.pap > 0.0)) {
-        // p has no component outside the null space of A^T (or r = 0): no step
-        c.alpha = 0.0;
+    if (!c.step) {
         c.active = 0;
         c.stalled = 1;
         return;
     }
-    c.alpha = c.rr / c.pap;
     c.rrnew = rn;
     if (!(sqrt(rn) < c.tol)) {
         if (rn > kCgGrowth * c.rrmin) {
@@ -818,7 +846,6 @@ __device__ __forceinline__ void cg_scalar_step(CgScalars& c, double pap, double 
             c.beta = rn / c.rr;
             c.rr = rn;
             c.rrmin = fmin(c.rrmin, rn);
-            c.do_p = 1;
             c.iter += 1;
             if (c.iter >= c.maxiter) c.active = 0;
         }
@@ -827,13 +854,17 @@ __device__ __forceinline__ void cg_scalar_step(CgScalars& c, double pap, double 
     }
     if (!isfinite(rn)) c.active = 0;
 }
+__device__ __forceinline__ void cg_scalar_rr(CgScalars& c, double rr) {
+    if (!c.active) return;
+    c.rr = rr;
+    c.rrmin = rr;
+}
 
-// One block per instance: r.r from the step kernel's partials (fixed tree),
-// then the scalars of cg_solver.cc:159-177: alpha, the ||r|| < tol test,
-// beta and the iteration count, the stops on p.Ap <= 0 and on residual
-// growth (kCgGrowth); counts the instances still iterating into n_active.
-__global__ void cg_beta_reduce_kernel(int nblk, int B, const double* __restrict__ partial,
-                                      const double* __restrict__ pap, CgScalars* cs, int* n_active) {
+// One block per instance: the sum of a map's per-CTA partials (fixed tree),
+// then the scalars: 0 the initial r.r, 1 q.q, 2 the new r.r, which also counts
+// the instances still iterating into n_active (cleared by 0 and 1).
+__global__ void cg_reduce_kernel(int what, int nblk, int B, const double* __restrict__ partial, CgScalars* cs,
+                                 int* n_active) {
     __shared__ double sh[kThreads];
     const int b = blockIdx.x;
     double s = 0.0;
@@ -846,232 +877,339 @@ __global__ void cg_beta_reduce_kernel(int nblk, int B, const double* __restrict_
     }
     if (threadIdx.x != 0) return;
     CgScalars c = cs[b];
-    cg_scalar_step(c, pap[b], sh[0]);
+    if (what == 0) {
+        cg_scalar_rr(c, sh[0]);
+    } else if (what == 1) {
+        cg_scalar_alpha(c, sh[0]);
+    } else {
+        cg_scalar_beta(c, sh[0]);
+        if (c.active) atomicAdd(n_active, 1);
+    }
+    if (what != 2 && b == 0) *n_active = 0;
     cs[b] = c;
-    if (c.active) atomicAdd(n_active, 1);
-}
-
-// One warp: per instance, test ||r|| < tol (cg_solver.cc:167-171), else beta
-// and iteration count; counts the instances still iterating.
-__global__ void cg_beta_kernel(int B, CgScalars* cs, const double* rrnew, int* n_active) {
-    int cnt = 0;
-    for (int b = threadIdx.x; b < B; b += blockDim.x) {
-        CgScalars c = cs[b];
-        c.do_p = 0;
-        if (c.active) {
-            const double rn = rrnew[b];
-            const double nrm = sqrt(rn);
-            c.rrnew = rn;
-            if (!(nrm < c.tol)) {
-                if (rn > kCgGrowth * c.rrmin) {
-                    // diverging on the null space of A^T: keep the current y (kernels.cuh)
-                    c.active = 0;
-                    c.stalled = 1;
-                } else {
-                    c.beta = rn / c.rr;
-                    c.rr = rn;
-                    c.rrmin = fmin(c.rrmin, rn);
-                    c.do_p = 1;
-                    c.iter += 1;
-                    if (c.iter >= c.maxiter) c.active = 0;
-                }
-            } else {
-                c.active = 0;
-            }
-            if (!isfinite(rn)) c.active = 0;
-        }
-        cnt += c.active;
-        cs[b] = c;
-    }
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    if (threadIdx.x == 0) *n_active = cnt;
-}
-
-__global__ void cg_update_p_kernel(int64_t n, int B, double* __restrict__ p, const double* __restrict__ r,
-                                   const CgScalars* __restrict__ cs) {
-    const int64_t total = n * B;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int b = (int)(t % B);
-        if (!cs[b].do_p) continue;
-        p[t] = cs[b].beta * p[t] + r[t];
-    }
 }
 
 // ---- persistent CG for small groups ------------------------------------------
 //
-// One cooperative launch runs a whole CG solve (cg_solver.cc:141-177) for a
-// group of at most kLoopMaxB instances: per iteration four phases over the
-// whole grid (A^T p; A (A^T p) with the per-unit partials of p.Ap; y += alpha
-// p and r -= alpha Ap with per-CTA partials of r.r; p = beta p + r),
-// separated by grid barriers.  Every CTA sums the partials itself in the same
-// fixed order, so every CTA holds the same scalars and takes the same
-// decision to continue; no CTA waits for a value only another CTA computes.
-// Vectors written inside the launch are read through L2 (ld.global.cg).
-// Each barrier wait is bounded: a wait that runs out sets *err and the CTA
-// leaves the kernel; the others then run out at their next wait.
+// One cooperative launch runs a whole CG solve for a group of at most
+// kLoopMaxB instances: q = A^T y and r = rhs - A q, then per iteration the two
+// passes of EpiCgQ and EpiCgR, each ended by an exchange of the CTAs' sums that
+// is also the grid's barrier.  Bound: the
+// exchanges and the latency of the gathers (the vectors sit in L2).  Every CTA
+// adds the posted sums itself in the same fixed order, so every CTA holds the same scalars and takes the same decision to continue; no CTA
+// waits for a value only another CTA computes.  Vectors written inside the
+// launch are read through L2 (ld.global.cg).  Each barrier wait is bounded: a
+// wait that runs out sets *err and the CTA leaves the kernel; the others then
+// run out at their next wait.
 
 constexpr long kGridWaitPolls = 1L << 25;  // about a second of polling (short sleeps)
-constexpr int kLoopCtasPerSm = 3;
 
 struct CgLoopArgs {
     DevMap A, AT;
     Blocks blA, blAT;  // unit layouts of the two maps
     int B;
-    int64_t nc;
-    double *y, *r, *p, *atp, *ap;
+    const double* rhs;
+    double *y, *r, *p, *q;
     CgScalars* cs;
-    double* part_dot;  // grid x B
-    double* part_rr;   // grid x B
-    unsigned int* bar;
+    unsigned long long* slots;  // three sets of grid x B
     int* err;
     int* n_active;
     int* iters;
     int cap;
 };
 
-// Arrive at barrier number target / gridDim.x of the launch and wait for all
-// CTAs; false when the wait ran out.
-__device__ __forceinline__ bool grid_wait(unsigned int* bar, unsigned int target, int* err) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        ok = 1;
-        // release: the CTA's writes (ordered before this by the barrier above)
-        // become visible to every CTA that acquires the counter
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-        unsigned int v = 0;
-        for (long n = 0;; n++) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-            if (v >= target) break;
-            if (n >= kGridWaitPolls) {
-                atomicExch(err, 1);
-                ok = 0;
-                break;
+// Grid barrier and per-instance sum in one: every CTA posts its value of each
+// instance (thread b < B holds instance b's) in its slot of the phase's set,
+// the CTA's threads wait for all the slots and add them (the same fixed order
+// in every CTA), then after(b, sum) runs in thread b.  A post is a release and
+// the poll an acquire, so what the CTAs wrote before is visible after.  Three
+// sets take turns: once a CTA has seen all posts of phase k, every CTA is done
+// with the set of phase k - 1, and the CTA empties its slots there before it
+// posts phase k + 1; the set is used again in phase k + 2.  Beside a counter
+// barrier and a pass over stored partials this saves a round trip to L2 per
+// phase.  The polls are spread over the CTA: a lane that polled 14 slots one
+// after the other took 13,000 cycles for it.  false when a wait ran out.
+// a slot per 128-byte line: packed side by side, 148 CTAs polling ten lines
+// took 11,000 cycles for an exchange, spread out 6,000
+constexpr int kSlotStride = 16;
+constexpr unsigned long long kSlotEmpty = ~0ull;  // cudaMemset(0xff): a NaN that no arithmetic here returns
+template <int MODE, class F>
+__device__ __forceinline__ bool grid_exchange(unsigned long long* sets, unsigned int& phase, int B, double v, int* err,
+                                              F&& after) {
+    const int G = (int)gridDim.x, n = G * B, t = (int)threadIdx.x;
+    unsigned long long* S = sets + (size_t)(phase % 3) * n * kSlotStride;
+    unsigned long long* prev = sets + (size_t)((phase + 2) % 3) * n * kSlotStride;
+    phase++;
+    __syncthreads();  // every thread's writes come before the posts
+    if (t < B) {
+        unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+        if (bits == kSlotEmpty) bits = 0x7ff8000000000000ull;  // a NaN all the same
+        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(S + ((size_t)blockIdx.x * B + t) * kSlotStride), "l"(bits) : "memory");
+    }
+    // thread t: instance t % B of CTAs t / B, t / B + T / B, ...
+    const int lanes = (int)blockDim.x / B * B;
+    double s = 0.0;
+    bool fine = true;
+    if (t < lanes) {
+        long polls = 0;
+        for (int k = t; k < n && fine; k += lanes) {
+            unsigned long long bits;
+            while (true) {
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(bits) : "l"(S + (size_t)k * kSlotStride) : "memory");
+                if (bits != kSlotEmpty) break;
+                if (++polls >= kGridWaitPolls) {
+                    atomicExch(err, 1);
+                    fine = false;
+                    break;
+                }
+                if (polls > 64) __nanosleep(32);
             }
-            if (n > 64) __nanosleep(32);
+            s += __longlong_as_double((long long)bits);
         }
     }
-    __syncthreads();
-    return ok != 0;
-}
-
-// out[b] = sum over k < n of part[k * B + b] for every instance b < B, the
-// same fixed order in every CTA (strided per thread, warp shuffles, warps).
-__device__ __forceinline__ void loop_reduce(const double* part, int n, int B, double* out) {
-    __shared__ double wsum[kThreads / 32][kLoopMaxB];
-    double acc[kLoopMaxB];
-#pragma unroll
-    for (int b = 0; b < kLoopMaxB; b++) acc[b] = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x)
-#pragma unroll
-        for (int b = 0; b < kLoopMaxB; b++)
-            if (b < B) acc[b] += __ldcg(part + (int64_t)k * B + b);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int b = 0; b < kLoopMaxB; b++) {
-        double v = acc[b];
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane == 0) wsum[warp][b] = v;
+    const double sum = MODE == kOne ? cta_sum(s) : cta_instance_sum(s, B);
+    if (t < B) {
+        prev[((size_t)blockIdx.x * B + t) * kSlotStride] = kSlotEmpty;
+        after(t, sum);
     }
-    __syncthreads();
-    if ((int)threadIdx.x < B) {
-        double t = 0.0;
-        for (int w = 0; w < kThreads / 32; w++) t += wsum[w][threadIdx.x];
-        out[threadIdx.x] = t;
-    }
-    __syncthreads();
+    return __syncthreads_and(fine) != 0;
 }
 
 template <int MODE, bool DEEP, bool PK>
-__global__ void __launch_bounds__(kThreads, kLoopCtasPerSm) cg_loop_kernel(const __grid_constant__ CgLoopArgs L) {
+__global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(const __grid_constant__ CgLoopArgs L) {
     __shared__ double bookA[kBookSize], bookAT[kBookSize];
     __shared__ CgScalars sc[kLoopMaxB];
-    __shared__ int sact[kLoopMaxB];
-    __shared__ double spap[kLoopMaxB], srn[kLoopMaxB];
-    __shared__ int s_any;
-    const int B = L.B;
+    const int B = MODE == kOne ? 1 : L.B;
+    const int b = (int)threadIdx.x;
     if (threadIdx.x < kBookSize) {
         bookA[threadIdx.x] = L.A.book[threadIdx.x];
         bookAT[threadIdx.x] = L.AT.book[threadIdx.x];
     }
-    if ((int)threadIdx.x < B) {
-        sc[threadIdx.x] = L.cs[threadIdx.x];
-        sact[threadIdx.x] = sc[threadIdx.x].active;
-    }
+    if (b < B) sc[b] = L.cs[b];
     __syncthreads();
-    const unsigned int G = gridDim.x;
-    unsigned int target = 0;
-    const EpiStore eAT{L.atp};
-    const EpiDot eA{L.p, L.ap};
+    unsigned int phase = 0;
+    struct EpiQ0 : EpiStore {  // q = A^T y where the instance is solved for
+        const CgScalars* cs;
+        __device__ __forceinline__ bool on(int i) const { return cs[i].active; }
+    } e0;
+    e0.out = L.q;
+    e0.mask = nullptr;
+    e0.cs = sc;
+    ell_cta<MODE, DEEP, false, PK, true>(L.AT, L.blAT, B, L.y, e0, bookAT);
+    if (!grid_exchange<MODE>(L.slots, phase, B, 0.0, L.err, [&](int, double) {})) return;
+    double s = ell_cta<MODE, DEEP, false, PK, true>(L.A, L.blA, B, L.q, EpiCgInit{sc, L.rhs, L.r}, bookA);
+    if (!grid_exchange<MODE>(L.slots, phase, B, s, L.err, [&](int i, double rr) { cg_scalar_rr(sc[i], rr); })) return;
     int it = 0;
-    while (true) {
-        if (threadIdx.x == 0) {
-            int a = 0;
-            for (int b = 0; b < B; b++) a |= sact[b];
-            s_any = a;
-        }
-        __syncthreads();
-        if (!s_any || it >= L.cap) break;
-        // A^T p
-        ell_cta<MODE, DEEP, false, PK, true>(L.AT, L.blAT, B, L.p, eAT, sact, bookAT);
-        target += G;
-        if (!grid_wait(L.bar, target, L.err)) return;
-        // Ap = A (A^T p) and the partials of p.Ap
-        {
-            const double s = ell_cta<MODE, DEEP, false, PK, true>(L.A, L.blA, B, L.atp, eA, sact, bookA);
-            if ((int)threadIdx.x < B) L.part_dot[(int64_t)blockIdx.x * B + threadIdx.x] = s;
-        }
-        target += G;
-        if (!grid_wait(L.bar, target, L.err)) return;
-        loop_reduce(L.part_dot, (int)G, B, spap);
-        // y += alpha p, r -= alpha Ap (cg_solver.cc:159-165), partials of r.r
-        {
-            const int rpp = kThreads / B, lanes = rpp * B;
-            const int b = threadIdx.x % B, rsub = threadIdx.x / B;
-            double acc = 0.0;
-            if ((int)threadIdx.x < lanes) {
-                const double pp = spap[b];
-                const bool act = sc[b].active && pp > 0.0;
-                const double a = act ? sc[b].rr / pp : 0.0;
-                for (int64_t e = (int64_t)blockIdx.x * rpp + rsub; e < L.nc; e += (int64_t)G * rpp) {
-                    const int64_t t = e * B + b;
-                    double rv = __ldcg(L.r + t);
-                    if (act) {
-                        L.y[t] = __ldcg(L.y + t) + a * __ldcg(L.p + t);
-                        rv += -a * __ldcg(L.ap + t);
-                        L.r[t] = rv;
-                    }
-                    acc += rv * rv;
-                }
-            }
-            block_partial(acc, B, L.part_rr, blockIdx.x);
-        }
-        target += G;
-        if (!grid_wait(L.bar, target, L.err)) return;
-        loop_reduce(L.part_rr, (int)G, B, srn);
-        if ((int)threadIdx.x < B) {
-            cg_scalar_step(sc[threadIdx.x], spap[threadIdx.x], srn[threadIdx.x]);
-            sact[threadIdx.x] = sc[threadIdx.x].active;
-        }
-        __syncthreads();
-        // p = beta p + r where the instance continues (cg_solver.cc:173-176)
-        for (int64_t t = (int64_t)blockIdx.x * kThreads + threadIdx.x; t < L.nc * B; t += (int64_t)G * kThreads) {
-            const int b = (int)(t % B);
-            if (!sc[b].do_p) continue;
-            L.p[t] = sc[b].beta * __ldcg(L.p + t) + __ldcg(L.r + t);
-        }
-        it++;
-        target += G;
-        if (!grid_wait(L.bar, target, L.err)) return;
+    for (; it < L.cap; it++) {
+        int any = 0;
+        for (int i = 0; i < B; i++) any |= sc[i].active;
+        if (!any) break;
+        s = ell_cta<MODE, DEEP, false, PK, true>(L.AT, L.blAT, B, L.r, EpiCgQ{sc, L.q}, bookAT);
+        if (!grid_exchange<MODE>(L.slots, phase, B, s, L.err, [&](int i, double qq) { cg_scalar_alpha(sc[i], qq); })) return;
+        s = ell_cta<MODE, DEEP, false, PK, true>(L.A, L.blA, B, L.q, EpiCgR{sc, L.y, L.r, L.p}, bookA);
+        if (!grid_exchange<MODE>(L.slots, phase, B, s, L.err, [&](int i, double rn) { cg_scalar_beta(sc[i], rn); })) return;
     }
     if (blockIdx.x == 0) {
-        if ((int)threadIdx.x < B) L.cs[threadIdx.x] = sc[threadIdx.x];
-        if (threadIdx.x == 0) {
+        if (b < B) L.cs[b] = sc[b];
+        if (b == 0) {
             int cnt = 0;
-            for (int b = 0; b < B; b++) cnt += sact[b];
+            for (int i = 0; i < B; i++) cnt += sc[i].active;
             *L.n_active = cnt;
             *L.iters = it;
+        }
+    }
+}
+
+// ---- resident CG --------------------------------------------------------------
+//
+// The persistent CG for groups small enough that every row of A and of A^T has
+// its own lanes: the table words and the row's elements of q, y, r and p stay
+// in registers for the whole solve, and an iteration's phase is one round of
+// gathers (through L2, where q and r are published), the sum over the CTA and
+// the exchange.  cg_loop_kernel instead reloads the row's words, its elements
+// and its output row each time, three L2 round trips of about 900 cycles in a
+// row (the acquire of each exchange drops the L1's lines); its slowest CTA
+// took 13,000 cycles for a phase at n = 10.  B200, us per CG iteration in a
+// solve, four counter barriers per iteration before and now: n = 4 34 -> 8.6,
+// n = 5 26.5 -> 8.9, n = 10 27.6 -> 11.5; a phase is about 2,000 cycles of
+// gathers and CTA sum and 3,700 (27 CTAs) to 6,000 (148) of exchange.
+constexpr int kResWords = 8;       // table words per lane
+constexpr int kResThreads = 1024;  // the largest CTA with one instance (64 registers), 768 with several (85)
+constexpr int kResClasses = kMaxBuckets + kLongClasses;
+constexpr int kResSmem = 2 * kResWords * kResThreads * (int)sizeof(int32_t);  // the words of both maps
+
+// One map's rows dealt to warps: class c has rows of up to 8 g[c] entries, g
+// lanes per row and instance (32 / (g B) rows per warp), from warp first[c].
+struct ResPlan {
+    int n, warps;
+    int first[kResClasses], g[kResClasses], rows[kResClasses];
+    int bucket[kResClasses];  // ELL bucket, or -1: long rows from row0
+    int row0[kResClasses];
+};
+
+struct CgResArgs {
+    DevMap A, AT;
+    ResPlan pA, pAT;
+    int B;
+    const double* rhs;
+    double *y, *r, *q;
+    CgScalars* cs;
+    unsigned long long* slots;  // three sets of grid x B
+    int* err;
+    int* n_active;
+    int* iters;
+    int cap;
+};
+
+// A thread's place in one map: its row and instance; its words are in shared
+// memory (in registers they spill, and the exchanges drop the L1's lines,
+// spilled ones too: eight reloads from L2 one after the other).
+struct ResLane {
+    int row, b, g, nw;  // row < 0: no row; nw: words in use (of any lane of the warp)
+    bool head;          // the lane that ends up with the row's sum
+};
+
+__device__ __forceinline__ ResLane res_load(const DevMap& M, const ResPlan& P, int warp, int B,
+                                            int32_t (*words)[kResThreads]) {
+    const int lane = threadIdx.x & 31;
+    ResLane L{-1, lane % B, 1, 0, false};
+    for (int j = 0; j < kResWords; j++) words[j][threadIdx.x] = -1;
+    if (warp >= P.warps) return L;
+    int c = 0;
+    while (c + 1 < P.n && warp >= P.first[c + 1]) c++;
+    const int gB = P.g[c] * B, rpw = 32 / gB, local = lane / gB, part = lane % gB / B;
+    const int slot = (warp - P.first[c]) * rpw + local;
+    const bool ok = local < rpw && slot < P.rows[c];
+    const int bi = P.bucket[c], k0 = part * kResWords;
+    L.g = P.g[c];
+    L.head = ok && part == 0;
+    L.nw = kResWords;
+    if (bi >= 0) {
+        const int W = M.width[bi];
+        if (W < kResWords) L.nw = W;
+        if (ok) {
+            L.row = M.rows[M.row_off[bi] + slot];
+            for (int j = 0; j < kResWords && k0 + j < W; j++)
+                words[j][threadIdx.x] = M.cols[M.ent_off[bi] + (int64_t)(k0 + j) * M.nslots[bi] + slot];
+        }
+    } else if (ok) {
+        const int m = P.row0[c] + slot;
+        const int at = M.res_ptr[m], len = M.res_ptr[m + 1] - at;
+        L.row = M.res_row[m];
+        for (int j = 0; j < kResWords && k0 + j < len; j++) words[j][threadIdx.x] = M.res_word[at + k0 + j];
+    }
+    return L;
+}
+
+// The row's sum (valid in the head lanes).
+__device__ __forceinline__ double res_gather(const double* in, const ResLane& L, int B,
+                                             const int32_t (*words)[kResThreads], const double* book) {
+    double s = 0.0;
+    for (int j0 = 0; j0 < L.nw; j0 += 4) {
+        int32_t w[4];
+        double g[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) w[j] = words[j0 + j][threadIdx.x];
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            g[j] = load_one<true>(in + (int64_t)(w[j] & ((1 << kCodeShift) - 1)) * B + L.b, w[j] >= 0);
+#pragma unroll
+        for (int j = 0; j < 4; j++) s += book[(w[j] >> kCodeShift) & (kBookSize - 1)] * g[j];
+    }
+    for (int h = L.g / 2; h > 0; h >>= 1) s += __shfl_down_sync(0xffffffffu, s, h * B);
+    return s;
+}
+
+template <bool ONE>
+__global__ void __launch_bounds__(ONE ? kResThreads : 768, 1) cg_resident_kernel(const __grid_constant__ CgResArgs A) {
+    __shared__ double bookA[kBookSize], bookAT[kBookSize];
+    __shared__ CgScalars sc[kLoopMaxB];
+    __shared__ double sums[kResThreads / 32 * kLoopMaxB];
+    const int B = ONE ? 1 : A.B;
+    const int t = (int)threadIdx.x;
+    if (t < kBookSize) {
+        bookA[t] = A.A.book[t];
+        bookAT[t] = A.AT.book[t];
+    }
+    if (t < B) sc[t] = A.cs[t];
+    const int warp = (t >> 5) * (int)gridDim.x + (int)blockIdx.x;
+    extern __shared__ int32_t res_words[];  // kResWords x kResThreads of each map
+    auto wx = reinterpret_cast<int32_t (*)[kResThreads]>(res_words), wc = wx + kResWords;
+    // this thread's row of A^T and of A
+    const ResLane lx = res_load(A.AT, A.pAT, warp, B, wx), lc = res_load(A.A, A.pA, warp, B, wc);
+    const int64_t tx = (int64_t)lx.row * B + lx.b, tc = (int64_t)lc.row * B + lc.b;
+    double y = 0.0, rhs = 0.0, r = 0.0, p = 0.0, q = 0.0;
+    if (lc.head) {
+        y = A.y[tc];
+        rhs = A.rhs[tc];
+    }
+    __syncthreads();
+    unsigned int phase = 0;
+    // per-instance sum of v over the CTA, to thread b
+    auto total = [&](double v) {
+        if (ONE) return cta_sum(v);
+        // lane l holds instance l % B: fold each warp, then the warps
+        const int lane = t & 31;
+        for (int left = 32 / B; left > 1;) {
+            const int h = (left + 1) / 2;
+            const double o = __shfl_down_sync(0xffffffffu, v, B * h);
+            if (lane / B < left - h) v += o;
+            left = h;
+        }
+        if (lane < B) sums[(t >> 5) * kLoopMaxB + lane] = v;
+        __syncthreads();
+        double s = 0.0;
+        if (t < B)
+            for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += sums[w * kLoopMaxB + t];
+        return s;
+    };
+    auto exchange = [&](double v, auto after) {
+        return grid_exchange<ONE ? kOne : kOdd>(A.slots, phase, B, v, A.err, after);
+    };
+    double s = res_gather(A.y, lx, B, wx, bookAT);  // q = A^T y
+    if (lx.head && sc[lx.b].active) A.q[tx] = s;
+    if (!exchange(0.0, [&](int, double) {})) return;
+    s = res_gather(A.q, lc, B, wc, bookA);  // r = rhs - A q
+    double v = 0.0;
+    if (lc.head && sc[lc.b].active) {
+        r = rhs - s;
+        A.r[tc] = r;
+        v = r * r;
+    }
+    if (!exchange(total(v), [&](int i, double rr) { cg_scalar_rr(sc[i], rr); })) return;
+    int it = 0;
+    for (; it < A.cap; it++) {
+        int any = 0;
+        for (int i = 0; i < B; i++) any |= sc[i].active;
+        if (!any) break;
+        s = res_gather(A.r, lx, B, wx, bookAT);
+        v = 0.0;
+        if (lx.head && sc[lx.b].active) {
+            q = s + sc[lx.b].beta * q;
+            A.q[tx] = q;
+            v = q * q;
+        }
+        if (!exchange(total(v), [&](int i, double qq) { cg_scalar_alpha(sc[i], qq); })) return;
+        s = res_gather(A.q, lc, B, wc, bookA);
+        v = 0.0;
+        if (lc.head && sc[lc.b].step) {
+            const double alpha = sc[lc.b].alpha;
+            p = r + sc[lc.b].beta * p;
+            y += alpha * p;
+            r -= alpha * s;
+            A.r[tc] = r;
+            v = r * r;
+        }
+        if (!exchange(total(v), [&](int i, double rn) { cg_scalar_beta(sc[i], rn); })) return;
+    }
+    if (lc.head) A.y[tc] = y;
+    if (blockIdx.x == 0) {
+        if (t < B) A.cs[t] = sc[t];
+        if (t == 0) {
+            int cnt = 0;
+            for (int i = 0; i < B; i++) cnt += sc[i].active;
+            *A.n_active = cnt;
+            *A.iters = it;
         }
     }
 }
@@ -1100,10 +1238,10 @@ static int map_threads(int B) {
     return std::max(kThreads / n * n, B) + 31 & ~31;
 }
 
-// Units of a map (Blocks).  Small maps (every tile resident at once with one
-// row per thread) keep one row per thread: there the kernel is one latency
-// chain, and more CTAs spread it wider.
-static Blocks map_blocks(const DevMap& M, int B, int threads) {
+// Units of a map (Blocks).  Small maps (at most deep_from tiles with one row per
+// thread, as many as are resident at once) keep one row per thread: there the
+// kernel is one latency chain, and more CTAs spread it wider.
+static Blocks map_blocks(const DevMap& M, int B, int threads, int deep_from) {
     Blocks bl{};
     const int64_t rpp = threads / lanes_of(B);
     auto tiles = [&](int i, bool deep) {
@@ -1112,7 +1250,7 @@ static Blocks map_blocks(const DevMap& M, int B, int threads) {
     };
     int64_t tot = 0;
     for (int i = 0; i < M.nb; i++) tot += tiles(i, false);
-    bl.deep = M.packed && tot > 148 * kMapCtasPerSm;
+    bl.deep = M.packed && tot > deep_from;
     bl.mid = M.nlong - M.nmid;
     bl.midchunks = (B + 31) / 32;
     const int warps = threads / 32;
@@ -1128,10 +1266,9 @@ static Blocks map_blocks(const DevMap& M, int B, int threads) {
 // Returns the partial sums written per instance (one per CTA, where the
 // epilogue sums).
 template <class Epi>
-static int run_map(const DevMap& M, int B, const double* in, const Epi& e, const int* mask, double* partial,
-                   cudaStream_t s) {
+static int run_map(const DevMap& M, int B, const double* in, const Epi& e, double* partial, cudaStream_t s) {
     const int threads = map_threads(B);
-    const Blocks bl = map_blocks(M, B, threads);
+    const Blocks bl = map_blocks(M, B, threads, 148 * kMapCtasPerSm);
     const int units = bl.start[kMaxBuckets];
     if (units == 0) return 0;
     // as many CTAs as fit on the device at once, each with its share of the units
@@ -1142,7 +1279,7 @@ static int run_map(const DevMap& M, int B, const double* in, const Epi& e, const
         auto k = bl.deep ? (st ? ell_kernel<MODE, true, true, true, Epi> : ell_kernel<MODE, true, false, true, Epi>)
                          : (M.packed ? ell_kernel<MODE, false, false, true, Epi>
                                      : ell_kernel<MODE, false, false, false, Epi>);
-        k<<<g, threads, 0, s>>>(M, bl, B, in, e, mask, partial);
+        k<<<g, threads, 0, s>>>(M, bl, B, in, e, partial);
     };
     switch (lane_mode(B)) {
         case kOne: go(std::integral_constant<int, kOne>()); break;
@@ -1156,19 +1293,12 @@ static int run_map(const DevMap& M, int B, const double* in, const Epi& e, const
 void launch_spmv(const DevMap& A, int B, const double* in, double* out, const double* sub, const double* coef,
                  const double* add, const int* mask, cudaStream_t s) {
     if (sub || coef || add)
-        run_map(A, B, in, EpiAffine{sub, coef, add, out}, mask, nullptr, s);
+        run_map(A, B, in, EpiAffine{sub, coef, add, out, mask}, nullptr, s);
     else
-        run_map(A, B, in, EpiStore{out}, mask, nullptr, s);
+        run_map(A, B, in, EpiStore{out, mask}, nullptr, s);
 }
 
 int64_t reduce_partial_size(int B) { return (int64_t)kSpmvBlocks * B; }
-
-void launch_spmv_dot(const DevMap& A, int B, const double* in, double* out, const double* dotv, const int* mask,
-                     double* partial, double* dot_out, cudaStream_t s) {
-    const int g = run_map(A, B, in, EpiDot{dotv, out}, mask, partial, s);
-    reduce_stage2<<<B, kThreads, 0, s>>>(g, B, partial, dot_out);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
 
 void launch_reduce(ReduceMode mode, int64_t n, int B, const double* u, const double* v, const double* w,
                    const double* row, double* partial, double* out, cudaStream_t s) {
@@ -1228,39 +1358,6 @@ void launch_c_minus_z(int64_t n, int B, const double* c, double* z, const int* m
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-void launch_cg_init(int64_t n, int B, const double* rhs, const double* Ap, double* r, double* p, const CgScalars* cs,
-                    cudaStream_t s) {
-    cg_init_kernel<<<grid_for(n * B), kThreads, 0, s>>>(n, B, rhs, Ap, r, p, cs);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
-void launch_cg_set_rr(int B, CgScalars* cs, const double* rr, int* n_active, cudaStream_t s) {
-    cg_set_rr_kernel<<<1, 32, 0, s>>>(B, cs, rr, n_active);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
-void launch_cg_alpha(int B, CgScalars* cs, const double* pap, cudaStream_t s) {
-    cg_alpha_kernel<<<(B + 127) / 128, 128, 0, s>>>(B, cs, pap);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
-void launch_cg_update_yr(int64_t n, int B, double* y, double* r, const double* p, const double* Ap,
-                         const CgScalars* cs, double* partial, double* rr_out, cudaStream_t s) {
-    const int g = spmv_grid(n, B);
-    cg_update_yr_kernel<<<g, kThreads, 0, s>>>(n, B, y, r, p, Ap, cs, partial);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-    reduce_stage2<<<B, kThreads, 0, s>>>(g, B, partial, rr_out);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
-void launch_cg_step(int64_t n, int B, double* y, double* r, const double* p, const double* Ap, CgScalars* cs,
-                    const double* pap, double* partial, int* n_active, cudaStream_t s) {
-    const int g = spmv_grid(n, B);
-    cg_step_yr_kernel<<<g, kThreads, 0, s>>>(n, B, y, r, p, Ap, cs, pap, partial, n_active);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-    cg_beta_reduce_kernel<<<B, kThreads, 0, s>>>(g, B, partial, pap, cs, n_active);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
-void launch_cg_beta(int B, CgScalars* cs, const double* rrnew, int* n_active, cudaStream_t s) {
-    cg_beta_kernel<<<1, 32, 0, s>>>(B, cs, rrnew, n_active);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
 // Condition of the device-side CG loop (the body of a WHILE node in the
 // group's CUDA graph): another iteration while an instance still iterates,
 // and never more than `cap` iterations in all.
@@ -1274,9 +1371,22 @@ void launch_cg_while(cudaGraphConditionalHandle h, const int* n_active, int* cou
     cg_while_kernel<<<1, 1, 0, s>>>(h, n_active, count, cap);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
-void launch_cg_update_p(int64_t n, int B, double* p, const double* r, const CgScalars* cs, cudaStream_t s) {
-    cg_update_p_kernel<<<grid_for(n * B), kThreads, 0, s>>>(n, B, p, r, cs);
+static void cg_reduce(int what, int nblk, int B, const double* partial, CgScalars* cs, int* n_active, cudaStream_t s) {
+    cg_reduce_kernel<<<B, kThreads, 0, s>>>(what, nblk, B, partial, cs, n_active);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+}
+
+void launch_cg_start(const DevMap& A, int B, const double* q, const double* rhs, double* r, CgScalars* cs,
+                     double* partial, int* n_active, cudaStream_t s) {
+    cg_reduce(0, run_map(A, B, q, EpiCgInit{cs, rhs, r}, partial, s), B, partial, cs, n_active, s);
+}
+void launch_cg_direction(const DevMap& AT, int B, const double* r, double* q, CgScalars* cs, double* partial,
+                         int* n_active, cudaStream_t s) {
+    cg_reduce(1, run_map(AT, B, r, EpiCgQ{cs, q}, partial, s), B, partial, cs, n_active, s);
+}
+void launch_cg_step(const DevMap& A, int B, const double* q, double* y, double* r, double* p, CgScalars* cs,
+                    double* partial, int* n_active, cudaStream_t s) {
+    cg_reduce(2, run_map(A, B, q, EpiCgR{cs, y, r, p}, partial, s), B, partial, cs, n_active, s);
 }
 
 int cg_loop_grid(int device) {
@@ -1289,10 +1399,14 @@ int cg_loop_grid(int device) {
     int g = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) == cudaSuccess && coop &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cg_loop_kernel<kOdd, true, true>, kThreads, 0) == cudaSuccess) {
-        // three CTAs per SM (the launch bound): the phases are latency-bound
-        // gathers that want the warps
-        const int per_sm = std::min(kLoopCtasPerSm, occ);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cg_loop_kernel<kOdd, true, true>, kLoopThreads, 0) == cudaSuccess &&
+        cudaFuncSetAttribute(cg_resident_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem) ==
+            cudaSuccess &&
+        cudaFuncSetAttribute(cg_resident_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem) ==
+            cudaSuccess) {
+        // one CTA per SM: an exchange costs by its CTAs (n = 10, one instance:
+        // 29.8 us per iteration with 430 CTAs of 256 threads)
+        const int per_sm = std::min(1, occ);
         if (per_sm >= 1) g = sms * per_sm;
     }
     cudaGetLastError();
@@ -1300,32 +1414,88 @@ int cg_loop_grid(int device) {
     return g;
 }
 
-bool cg_loop_fits(int64_t nc, int B) { return B >= 1 && B <= kLoopMaxB && nc * B <= kLoopMaxElems; }
+size_t cg_loop_slots(int grid, int B) { return 3 * (size_t)grid * B * kSlotStride; }
 
-cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, int64_t nc, double* y, double* r, double* p,
-                           double* atp, double* ap, CgScalars* cs, double* part_dot, double* part_rr,
-                           unsigned int* bar, int* err, int* n_active, int* iters, int cap, int grid,
-                           cudaStream_t s) {
+bool cg_loop_fits(int64_t nc, int B) { return B >= 1 && B <= kLoopMaxB && nc <= kLoopMaxRows; }
+
+// The rows of M dealt to warps for B instances; false when they do not fit
+// (unpacked, or rows longer than 8 entries for each of 32 / B lanes).
+static bool res_plan(const DevMap& M, int B, ResPlan& P) {
+    if (M.nres < 0) return false;
+    P = ResPlan{};
+    int64_t at = 0;
+    auto add = [&](int g, int64_t rows, int bucket, int row0) {
+        if (rows == 0) return true;
+        if (g * B > 32 || P.n == kResClasses) return false;
+        const int rpw = 32 / (g * B);
+        P.first[P.n] = (int)at;
+        P.g[P.n] = g;
+        P.rows[P.n] = (int)rows;
+        P.bucket[P.n] = bucket;
+        P.row0[P.n] = row0;
+        P.n++;
+        at += (rows + rpw - 1) / rpw;
+        return at < (1 << 24);
+    };
+    for (int i = 0; i < M.nb; i++)
+        if (!add(std::max(1, M.width[i] / kResWords), M.nslots[i], i, 0)) return false;
+    // the long rows, sorted by length
+    int row0 = 0;
+    for (int c = 0; c < kLongClasses; c++) {
+        if (!add(2 << c, M.res_upto[c] - row0, -1, row0)) return false;
+        row0 = M.res_upto[c];
+    }
+    P.warps = (int)at;
+    return true;
+}
+
+static bool cg_resident(const DevMap& A, const DevMap& AT, int B, int sms, ResPlan& pA, ResPlan& pAT, int& grid,
+                        int& threads) {
+    if (!res_plan(A, B, pA) || !res_plan(AT, B, pAT)) return false;
+    const int warps = std::max(pA.warps, pAT.warps);
+    // eight warps per CTA while the device has SMs for them
+    grid = std::min(sms, std::max(1, (warps + 7) / 8));
+    threads = 32 * ((warps + grid - 1) / grid);
+    return threads <= (B == 1 ? kResThreads : 768);
+}
+
+cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, const double* rhs, double* y, double* r, double* p,
+                           double* q, CgScalars* cs, unsigned long long* slots, int* err, int* n_active,
+                           int* iters, int cap, int grid, cudaStream_t s) {
+    cudaError_t e;
+    ResPlan pA, pAT;
+    int rgrid = 0, rthreads = 0;
+    if (cg_resident(A, AT, B, grid, pA, pAT, rgrid, rthreads)) {
+        e = cudaMemsetAsync(slots, 0xff, cg_loop_slots(rgrid, B) * sizeof(*slots), s);
+        if (e != cudaSuccess) return e;
+        CgResArgs R{A, AT, pA, pAT, B, rhs, y, r, q, cs, slots, err, n_active, iters, cap};
+        void* args[] = {&R};
+        const void* fn = B == 1 ? (const void*)cg_resident_kernel<true> : (const void*)cg_resident_kernel<false>;
+        e = cudaLaunchCooperativeKernel(fn, dim3(rgrid), dim3(rthreads), args, kResSmem, s);
+        g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+        return e;
+    }
     CgLoopArgs L;
     L.A = A;
     L.AT = AT;
-    L.blA = map_blocks(L.A, B, kThreads);
-    L.blAT = map_blocks(L.AT, B, kThreads);
+    L.blA = map_blocks(L.A, B, kLoopThreads, 4 * grid);
+    L.blAT = map_blocks(L.AT, B, kLoopThreads, 4 * grid);
+    // no more CTAs than the larger map has units: a barrier costs by its CTAs
+    grid = std::min(grid, std::max(L.blA.start[kMaxBuckets], L.blAT.start[kMaxBuckets]));
     L.B = B;
-    L.nc = nc;
+    L.rhs = rhs;
     L.y = y;
     L.r = r;
     L.p = p;
-    L.atp = atp;
-    L.ap = ap;
+    L.q = q;
     L.cs = cs;
-    L.part_dot = part_dot;
-    L.part_rr = part_rr;
-    L.bar = bar;
+    L.slots = slots;
     L.err = err;
     L.n_active = n_active;
     L.iters = iters;
     L.cap = cap;
+    e = cudaMemsetAsync(slots, 0xff, cg_loop_slots(grid, B) * sizeof(*slots), s);
+    if (e != cudaSuccess) return e;
     void* args[] = {&L};
     auto pick = [&](auto mode) -> const void* {
         constexpr int MODE = decltype(mode)::value;
@@ -1337,7 +1507,7 @@ cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, int64_t nc,
     const void* fn = lm == kOne ? pick(std::integral_constant<int, kOne>())
                                 : (lm == kOdd ? pick(std::integral_constant<int, kOdd>())
                                               : pick(std::integral_constant<int, kEven>()));
-    const cudaError_t e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, 0, s);
+    e = cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kLoopThreads), args, 0, s);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     return e;
 }

@@ -96,7 +96,7 @@ struct DevBuf {
 
 // One map (A or A^T) on the device in the bucketed-ELL form of kernels.cuh.
 struct MapTable {
-    DevBuf<int32_t> rows, cols, long_rows, long_ptr, long_col;
+    DevBuf<int32_t> rows, cols, long_rows, long_ptr, long_col, res_row, res_ptr, res_word;
     DevBuf<double> vals, long_val;
     DevMap dm;
 
@@ -104,8 +104,8 @@ struct MapTable {
     // columns fit in kCodeShift bits and the table has at most kBookSize
     // distinct coefficients (compared bit for bit, so the sums are unchanged);
     // returns the book, or an empty vector when the table stays unpacked.
-    static std::vector<double> pack(std::vector<int32_t>& hcols, const std::vector<double>& hvals) {
-        std::map<uint64_t, int> code;
+    static std::vector<double> pack(std::vector<int32_t>& hcols, const std::vector<double>& hvals,
+                                    std::map<uint64_t, int>& code) {
         std::vector<double> bk;
         for (size_t k = 0; k < hcols.size(); k++) {
             if (hcols[k] < 0) continue;
@@ -128,6 +128,44 @@ struct MapTable {
         return bk;
     }
 
+    // The long rows for the resident CG: sorted by length, entries packed with
+    // the same book, which takes up their coefficients too; left out when the
+    // book or the 256 entries of a row do not hold them.
+    void pack_long(const Csr& M, std::vector<int32_t> order, std::map<uint64_t, int>& code, std::vector<double>& bk) {
+        int used = (int)code.size();
+        std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
+            return M.rowptr[a + 1] - M.rowptr[a] < M.rowptr[b + 1] - M.rowptr[b];
+        });
+        std::vector<int32_t> ptr(1, 0), word;
+        for (int32_t r : order) {
+            if (M.rowptr[r + 1] - M.rowptr[r] > 256) return;
+            for (int64_t k = M.rowptr[r]; k < M.rowptr[r + 1]; k++) {
+                uint64_t bits;
+                std::memcpy(&bits, &M.val[k], sizeof bits);
+                auto it = code.find(bits);
+                if (it == code.end()) {
+                    if (used == kBookSize) return;
+                    bk[used] = M.val[k];
+                    it = code.emplace(bits, used++).first;
+                }
+                if (M.col[k] >= (1 << kCodeShift)) return;
+                word.push_back(M.col[k] | it->second << kCodeShift);
+            }
+            ptr.push_back((int32_t)word.size());
+        }
+        dm.nres = (int)order.size();
+        for (int c = 0, at = 0; c < kLongClasses; c++) {
+            while (at < dm.nres && M.rowptr[order[at] + 1] - M.rowptr[order[at]] <= (16 << c)) at++;
+            dm.res_upto[c] = at;
+        }
+        res_row.upload(order.data(), order.size());
+        res_ptr.upload(ptr.data(), ptr.size());
+        res_word.upload(word.data(), word.size());
+        dm.res_row = res_row.p;
+        dm.res_ptr = res_ptr.p;
+        dm.res_word = res_word.p;
+    }
+
     void build(const Csr& M) {
         static const int widths[kMaxBuckets] = {1, 2, 4, 5, 8, 16, 32};
         std::vector<std::vector<int32_t>> brow(kMaxBuckets);
@@ -137,6 +175,7 @@ struct MapTable {
             const int64_t len = M.rowptr[r + 1] - M.rowptr[r];
             int w = 0;
             while (w < kMaxBuckets && widths[w] < len) w++;
+            if (M.nrows < kLatencyRows && len > 16) w = kMaxBuckets;
             if (w < kMaxBuckets) {
                 brow[w].push_back((int32_t)r);
             } else {
@@ -151,7 +190,7 @@ struct MapTable {
         for (int32_t r : lrows) same[M.rowptr[r + 1] - M.rowptr[r]]++;
         const auto mid_end = std::stable_partition(lrows.begin(), lrows.end(), [&](int32_t r) {
             const int64_t len = M.rowptr[r + 1] - M.rowptr[r];
-            return len <= kMidRow && same[len] >= kMidMany;
+            return len <= kMidRow && (same[len] >= kMidMany || len <= 32);
         });
         for (int32_t r : lrows) {
             for (int64_t k = M.rowptr[r]; k < M.rowptr[r + 1]; k++) {
@@ -195,10 +234,12 @@ struct MapTable {
                 }
             }
         }
-        const std::vector<double> bk = pack(hcols, hvals);
+        std::map<uint64_t, int> code;
+        std::vector<double> bk = pack(hcols, hvals, code);
         rows.upload(hrows.data(), hrows.size());
         cols.upload(hcols.data(), hcols.size());
         if (bk.empty()) vals.upload(hvals.data(), hvals.size());
+        if (!bk.empty()) pack_long(M, lrows, code, bk);
         long_rows.upload(lrows.data(), lrows.size());
         long_ptr.upload(lptr.data(), lptr.size());
         long_col.upload(lcol.data(), lcol.size());
@@ -337,7 +378,6 @@ class GroupRun {
         bv_.alloc(C);
         r_.alloc(C);
         p_.alloc(C);
-        ap_.alloc(C);
         partial_.alloc(reduce_partial_size(B_) + (int64_t)(T.max_long() + 8) * B_);
         red_.alloc(4 * B_);
         mu_.alloc(B_);
@@ -364,8 +404,8 @@ class GroupRun {
         tune_maps();
         if (cg_loop_fits(nc_, B_)) loop_grid_ = cg_loop_grid(T.device);
         if (loop_grid_ > 0) {
-            loopbar_.alloc(2);
-            looppart_.alloc((size_t)loop_grid_ * B_);
+            looperr_.alloc(1);
+            loopslots_.alloc(cg_loop_slots(loop_grid_, B_));
         }
         alloc_anderson(X);
         if (const char* d = std::getenv("V2G_DIAG")) diag_every_ = std::atoi(d);
@@ -1121,16 +1161,9 @@ class GroupRun {
         }
     }
 
-    // CG map launch with optional CUDA-event timing (profile mode).
-    // With dotv, also red_[b] = sum dotv[., b] * out[., b].
-    void map_launch(const DevMap& M, const double* in, double* out, const double* dotv = nullptr,
-                    const int* mask = nullptr) {
-        auto go = [&]() {
-            if (dotv)
-                launch_spmv_dot(M, B_, in, out, dotv, mask, partial_.p, red_.p, s_);
-            else
-                launch_spmv(M, B_, in, out, nullptr, nullptr, nullptr, mask, s_);
-        };
+    // A map launch of the CG with optional CUDA-event timing (profile mode).
+    template <class F>
+    void timed(const DevMap& M, F&& go) {
         if (!profile_) {
             go();
             return;
@@ -1155,31 +1188,26 @@ class GroupRun {
     }
     // CGSolver::solve for every instance whose CG scalars are active.
     void cg_solve() {
-        // Ap = A A^T y ; r = B - Ap ; p = r
-        map_launch(mAT_, y_.p, atp_.p, nullptr, mask_.p);
-        map_launch(mA_, atp_.p, ap_.p, nullptr, mask_.p);
-        launch_cg_init(nc_, B_, bv_.p, ap_.p, r_.p, p_.p, cs_.p, s_);
-        launch_reduce(RED_DOT, nc_, B_, r_.p, r_.p, nullptr, nullptr, partial_.p, red_.p, s_);
-        launch_cg_set_rr(B_, cs_.p, red_.p, nact_.p, s_);
         // Small groups (outside profile mode): the whole solve in one
         // cooperative launch, the phases of each iteration separated by grid
-        // barriers (maps.cu), one host synchronisation per solve
+        // exchanges (maps.cu), one host synchronisation per solve
         if (!profile_ && loop_grid_ > 0) {
             int cap = 1;
             for (auto* p : P_) cap = std::max(cap, p->opt.cg_maxiter);
             cap += 2;
-            CK(cudaMemsetAsync(loopbar_.p, 0, 2 * sizeof(unsigned int), s_));
-            CK(launch_cg_loop(mA_, mAT_, B_, nc_, y_.p, r_.p, p_.p, atp_.p, ap_.p, cs_.p, partial_.p, looppart_.p,
-                              loopbar_.p, reinterpret_cast<int*>(loopbar_.p + 1), nact_.p, nact_.p + 6, cap,
-                              loop_grid_, s_));
+            CK(launch_cg_loop(mA_, mAT_, B_, bv_.p, y_.p, r_.p, p_.p, atp_.p, cs_.p, loopslots_.p, looperr_.p,
+                              nact_.p, nact_.p + 6, cap, loop_grid_, s_));
             CK(cudaMemcpyAsync(hnact_, nact_.p, sizeof(int), cudaMemcpyDeviceToHost, s_));
             CK(cudaMemcpyAsync(hnact_ + 6, nact_.p + 6, sizeof(int), cudaMemcpyDeviceToHost, s_));
-            CK(cudaMemcpyAsync(hnact_ + 7, loopbar_.p + 1, sizeof(int), cudaMemcpyDeviceToHost, s_));
+            CK(cudaMemcpyAsync(hnact_ + 7, looperr_.p, sizeof(int), cudaMemcpyDeviceToHost, s_));
             CK(cudaStreamSynchronize(s_));
-            if (hnact_[7] != 0) throw CudaError("a grid barrier of the persistent CG did not complete (wait ran out)");
+            if (hnact_[7] != 0) throw CudaError("an exchange of the persistent CG did not complete (wait ran out)");
             cg_loop_iters_ += hnact_[6];
-            if (hnact_[0] == 0) return;
+            return;  // cap iterations stop every instance by its own CG_MAXITER
         }
+        // q = A^T y, r = rhs - A q
+        timed(mAT_, [&] { launch_spmv(mAT_, B_, y_.p, atp_.p, nullptr, nullptr, nullptr, mask_.p, s_); });
+        timed(mA_, [&] { launch_cg_start(mA_, B_, atp_.p, bv_.p, r_.p, cs_.p, partial_.p, nact_.p, s_); });
         // Outside profile mode the iterations run as a device-side loop: a
         // CUDA graph (captured once per group) whose WHILE node repeats one
         // CG iteration until no instance iterates, bounded by the largest
@@ -1220,10 +1248,8 @@ class GroupRun {
     static constexpr int kCgChunk = 4;
     // One CG iteration (cg_solver.cc:141-177) for every instance whose scalars are active.
     void cg_iteration() {
-        map_launch(mAT_, p_.p, atp_.p, nullptr, mask_.p);
-        map_launch(mA_, atp_.p, ap_.p, p_.p, mask_.p);  // Ap and p.Ap (into red_)
-        launch_cg_step(nc_, B_, y_.p, r_.p, p_.p, ap_.p, cs_.p, red_.p, partial_.p, nact_.p, s_);
-        launch_cg_update_p(nc_, B_, p_.p, r_.p, cs_.p, s_);
+        timed(mAT_, [&] { launch_cg_direction(mAT_, B_, r_.p, atp_.p, cs_.p, partial_.p, nact_.p, s_); });
+        timed(mA_, [&] { launch_cg_step(mA_, B_, atp_.p, y_.p, r_.p, p_.p, cs_.p, partial_.p, nact_.p, s_); });
     }
     // kCgChunk CG iterations captured from the stream into a graph: the
     // kernels' arguments are the group's fixed buffers, so one capture serves
@@ -1483,7 +1509,7 @@ class GroupRun {
     cudaStream_t s_ = nullptr;
     cudaStream_t s_small_ = nullptr;  // the small blocks' projection, beside the large blocks'
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
-    DevBuf<double> c_, x_, z_, aty_, atp_, y_, ax_, bv_, r_, p_, ap_, partial_, red_, mu_, coef_;
+    DevBuf<double> c_, x_, z_, aty_, atp_, y_, ax_, bv_, r_, p_, partial_, red_, mu_, coef_;
     DevBuf<int> mask_, nact_, smask1_, smask2_;
     DevBuf<CgScalars> cs_;
     // CG start extrapolation (cg_extrapolate): the previous CG start and the
@@ -1538,10 +1564,10 @@ class GroupRun {
     cudaGraphExec_t cg_exec_ = nullptr;
     long cg_chunk_nodes_ = 0;
     // the persistent CG (small groups): cooperative grid size (0: not used),
-    // barrier counter and error flag, per-CTA partials of r.r
+    // slots of the CTAs' sums, error flag
     int loop_grid_ = 0;
-    DevBuf<unsigned int> loopbar_;
-    DevBuf<double> looppart_;
+    DevBuf<unsigned long long> loopslots_;
+    DevBuf<int> looperr_;
     long cg_loop_iters_ = 0;
     cudaGraphExec_t cg_loop_exec_ = nullptr;  // the device-side CG loop (WHILE node)
     long cg_loop_nodes_ = 0;
