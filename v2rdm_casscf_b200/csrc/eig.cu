@@ -3,12 +3,10 @@
 // For every primal block the reference symmetrises U = mu x + A^T y - c,
 // diagonalises it (Matrix::diagonalize) and rebuilds x = V+ (L+/mu) V+^T and
 // z = -V- L- V-^T.  Here:
-//   * blocks with n <= 64 are diagonalised by a parallel cyclic Jacobi method
-//     in shared memory, one CTA per block, and x and z are rebuilt in the same
-//     kernel;
+//   * blocks with n <= 64 take the matrix sign in shared memory (psd_sign.cu);
 //   * larger blocks use a two-sided block Jacobi method on a workspace padded
 //     to a multiple of 64: each round pairs 32-wide column blocks, solves the
-//     64 x 64 pair problems with the same shared-memory Jacobi, and rotates the
+//     64 x 64 pair problems with a shared-memory Jacobi, and rotates the
 //     workspace W and the eigenvector matrix V tile by tile.  The eigenvectors
 //     of the previous outer iteration seed the next one (W = V^T U V), so a
 //     warm solve needs one or two sweeps.  x = V diag(max(L,0)/mu) V^T and
@@ -172,91 +170,7 @@ __device__ void jacobi_smem(double* A, double* V, int N, int max_sweeps, double 
 }
 
 constexpr double kJacobiRotEps = 1e-15;
-constexpr int kJacobiSweeps = 20;
 constexpr int kPairSweeps = 1;
-
-// vsave (optional): the block's eigenvectors, n x n at t.woff, kept across
-// outer iterations.  With warm set, the Jacobi starts from them: A <- V^T U V
-// (nearly diagonal once the iteration settles, so one to three sweeps
-// converge it instead of ~10 from the identity) and the rotations accumulate
-// onto V.  Without warm the Jacobi starts from V = I; vsave is written either way.
-__global__ void __launch_bounds__(kJThreads) small_project_kernel(const BlockTask* __restrict__ tasks, int B,
-                                                                  const double* __restrict__ aty,
-                                                                  const double* __restrict__ c, double* x, double* z,
-                                                                  const double* __restrict__ mu,
-                                                                  const int* __restrict__ mask,
-                                                                  double* __restrict__ vsave, int warm,
-                                                                  const double* __restrict__ stol) {
-    extern __shared__ double sm[];
-    double* A = sm;
-    double* V = sm + kJ * kLd;
-    double* T = sm + 2 * kJ * kLd;  // only with vsave (the launch then has room for it)
-    const BlockTask t = tasks[blockIdx.x];
-    const int b = t.inst;
-    if (mask && !mask[b]) return;
-    const int N = t.n;
-    const double m = mu[b];
-    for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
-        const int p = i / N, q = i % N;
-        const int64_t e1 = (t.xoff + (int64_t)p * N + q) * B + b;
-        const int64_t e2 = (t.xoff + (int64_t)q * N + p) * B + b;
-        const double t1 = (aty[e1] - c[e1]) + m * x[e1];
-        const double t2 = (aty[e2] - c[e2]) + m * x[e2];
-        A[p * kLd + q] = 0.5 * (t1 + t2);
-    }
-    const bool use_warm = vsave && warm;
-    if (use_warm) {
-        const double* vs = vsave + t.woff;
-        for (int i = threadIdx.x; i < N * N; i += blockDim.x) V[(i / N) * kLd + (i % N)] = vs[i];
-        __syncthreads();
-        // T = A V, then A = V^T T (symmetrised)
-        for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
-            const int p = i / N, q = i % N;
-            double acc = 0.0;
-            for (int k = 0; k < N; k++) acc += A[p * kLd + k] * V[k * kLd + q];
-            T[p * kLd + q] = acc;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
-            const int p = i / N, q = i % N;
-            double acc = 0.0;
-            for (int k = 0; k < N; k++) acc += V[k * kLd + p] * T[k * kLd + q];
-            A[p * kLd + q] = acc;
-        }
-        __syncthreads();
-        for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
-            const int p = i / N, q = i % N;
-            if (p < q) {
-                const double v = 0.5 * (A[p * kLd + q] + A[q * kLd + p]);
-                A[p * kLd + q] = v;
-                A[q * kLd + p] = v;
-            }
-        }
-    }
-    __syncthreads();
-    // with stol, off-diagonal entries below the instance's share of the
-    // adaptive tolerance are left (x and z stay PSD; the residual is bounded)
-    jacobi_smem(A, V, N, kJacobiSweeps, kJacobiRotEps, !use_warm, stol ? stol[b] : 0.0);
-    __syncthreads();
-    if (vsave) {
-        double* vs = vsave + t.woff;
-        for (int i = threadIdx.x; i < N * N; i += blockDim.x) vs[i] = V[(i / N) * kLd + (i % N)];
-    }
-    for (int i = threadIdx.x; i < N * N; i += blockDim.x) {
-        const int p = i / N, q = i % N;
-        double sx = 0.0, sz = 0.0;
-        for (int j = 0; j < N; j++) {
-            const double lam = A[j * kLd + j];
-            if (lam > 0.0)
-                sx += (V[p * kLd + j] * lam / m) * V[q * kLd + j];
-            else if (lam < 0.0)
-                sz += (-V[p * kLd + j] * lam) * V[q * kLd + j];
-        }
-        const int64_t e = (t.xoff + (int64_t)p * N + q) * B + b;
-        x[e] = sx;
-        z[e] = sz;
-    }
-}
 
 // ---- large blocks ----------------------------------------------------------
 
@@ -1077,7 +991,6 @@ __global__ void write_xz_kernel(const BlockTask* __restrict__ tasks, int B, cons
 }
 
 constexpr size_t kJacobiSmem = 2 * kJ * kLd * sizeof(double);
-constexpr size_t kJacobiWarmSmem = 3 * kJ * kLd * sizeof(double);  // + the T of a warm start
 
 // The 66,560 B of dynamic shared memory of the Jacobi kernels need an opt-in
 // per kernel and per device.  Each device is set up once; a failed attempt is
@@ -1089,9 +1002,7 @@ void set_smem_attrs() {
     static std::vector<char> done;
     std::lock_guard<std::mutex> lk(mu);
     if ((size_t)dev < done.size() && done[dev]) return;
-    bool ok = cudaFuncSetAttribute(small_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)kJacobiWarmSmem) == cudaSuccess;
-    ok = ok && cudaFuncSetAttribute(bj_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    bool ok = cudaFuncSetAttribute(bj_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kJacobiSmem) == cudaSuccess;
     ok = ok && cudaFuncSetAttribute(bj_update_wv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kJacobiSmem) == cudaSuccess;
@@ -1101,16 +1012,6 @@ void set_smem_attrs() {
 }
 
 }  // namespace
-
-void launch_small_project(const BlockTask* tasks, int ntasks, int B, const double* aty, const double* c, double* x,
-                          double* z, const double* mu, const int* mask, cudaStream_t s, double* vsave, bool warm,
-                          const double* stol) {
-    if (ntasks == 0) return;
-    set_smem_attrs();
-    small_project_kernel<<<ntasks, kJThreads, vsave ? kJacobiWarmSmem : kJacobiSmem, s>>>(
-        tasks, B, aty, c, x, z, mu, mask, vsave, warm ? 1 : 0, stol);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
 
 void launch_form_u(const BlockTask* tasks, int ntasks, int max_np, int B, const double* aty, const double* c,
                       const double* x, const double* mu, const int* mask, double* Uw, cudaStream_t s) {

@@ -482,20 +482,14 @@ class GroupRun {
         // The small blocks (one CTA each: a few SMs for a few hundred
         // microseconds) run on a second stream beside the large blocks' path;
         // both read A^T y, c and mu and write disjoint entries of x and z.
-        // They start from their previous eigenvectors, except in the first
-        // projection, after a cold restart and every kSmallCold-th projection
-        // (so that rounding in the kept eigenvectors cannot build up).
-        const bool small_warm = small_warm_ && (nproj_ % kSmallCold) != 0;
         const bool fork = nsmall_ > 0;
         if (fork) {
             CK(cudaEventRecord(ev_fork_, s_));
             CK(cudaStreamWaitEvent(s_small_, ev_fork_, 0));
-            launch_small_project(small_d_.p, nsmall_, B_, aty_.p, c_.p, x_.p, z_.p, mu_.p, mask_.p, s_small_,
-                                 vsmall_.p, small_warm);
+            launch_small_project(small_d_.p, nsmall_, max_small_, B_, aty_.p, c_.p, x_.p, z_.p, mu_.p, mask_.p,
+                                 s_small_, small_hint_.p);
             CK(cudaEventRecord(ev_join_, s_small_));
         }
-        small_warm_ = true;
-        nproj_++;
         project_large(rho);
         if (fork) CK(cudaStreamWaitEvent(s_, ev_join_, 0));
     }
@@ -703,7 +697,6 @@ class GroupRun {
                         aa.restart(b);
                     }
                 warm_ = false;  // every block of the group starts its projection cold again
-                small_warm_ = false;
             }
             int nactive = 0;
             for (int b = 0; b < B_; b++) nactive += active[b];
@@ -1354,7 +1347,7 @@ class GroupRun {
     void build_projection_plan() {
         const Layout& L = T_.L;
         std::vector<BlockTask> small;
-        int64_t woff = 0, qoff = 0, doff = 0, soff = 0;
+        int64_t woff = 0, qoff = 0, doff = 0;
         for (int b = 0; b < B_; b++)
             for (size_t k = 0; k < L.block_dims.size(); k++) {
                 const int n = L.block_dims[k];
@@ -1364,8 +1357,7 @@ class GroupRun {
                 t.n = n;
                 t.inst = b;
                 if (n <= 64) {
-                    t.woff = soff;  // its kept eigenvectors
-                    soff += (int64_t)n * n;
+                    max_small_ = std::max(max_small_, n);
                     small.push_back(t);
                     continue;
                 }
@@ -1382,7 +1374,7 @@ class GroupRun {
         nsmall_ = (int)small.size();
         nlarge_ = (int)hlarge_.size();
         small_d_.upload(small.data(), small.size());
-        vsmall_.alloc(std::max<int64_t>(soff, 1));
+        small_hint_.alloc(small.size());
         large_d_.upload(hlarge_.data(), hlarge_.size());
         if (nlarge_ == 0) return;
         U_.alloc(woff);
@@ -1554,11 +1546,9 @@ class GroupRun {
     DevBuf<VTileTask> vtiles_;
     int ngtiles_ = 0, nstiles_ = 0, npairs_ = 0, nwtiles_ = 0, nvtiles_ = 0;
     bool warm_ = false;
-    // kept eigenvectors of the small blocks (warm Jacobi starts)
-    static constexpr long kSmallCold = 64;
-    DevBuf<double> vsmall_;
-    bool small_warm_ = false;
-    long nproj_ = 0;
+    // the small blocks' lift counts of the previous projection
+    int max_small_ = 0;
+    DevBuf<int> small_hint_;
     long sweeps_total_ = 0;
     // the captured CG chunk
     cudaGraphExec_t cg_exec_ = nullptr;
@@ -2246,6 +2236,7 @@ int v2g_update_xz_noalloc(v2g_handle* h, double mu, const double* d_c, const dou
         NoAllocSetup setup{};
         setup.mu = mu;
         setup.nt = 0;
+        int max_n = 0;
         for (size_t k = 0; k < L.block_dims.size(); k++) {
             const int n = L.block_dims[k];
             if (n == 0) continue;
@@ -2255,6 +2246,7 @@ int v2g_update_xz_noalloc(v2g_handle* h, double mu, const double* d_c, const dou
             if (setup.nt == kNoAllocMaxTasks)
                 return v2g::fail(V2G_ERR_ARG, "v2g_update_xz_noalloc: more than " +
                                                   std::to_string(kNoAllocMaxTasks) + " blocks");
+            max_n = std::max(max_n, n);
             setup.n[setup.nt] = n;
             setup.xoff[setup.nt] = L.block_off[k];
             setup.nt++;
@@ -2271,7 +2263,7 @@ int v2g_update_xz_noalloc(v2g_handle* h, double mu, const double* d_c, const dou
         v2g::g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
         CK(cudaMemsetAsync(s_aty, 0, L.dimx * sizeof(double), s));
         v2g::launch_spmv(T.AT(), 1, d_y, s_aty, nullptr, nullptr, nullptr, nullptr, s);
-        v2g::launch_small_project(s_tasks, setup.nt, 1, s_aty, d_c, d_x, d_z, s_mu, nullptr, s);
+        v2g::launch_small_project(s_tasks, setup.nt, max_n, 1, s_aty, d_c, d_x, d_z, s_mu, nullptr, s);
         CK(cudaGetLastError());
         return V2G_OK;
     });
