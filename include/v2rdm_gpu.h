@@ -60,10 +60,10 @@ typedef struct v2g_options {
     int device;                 /* CUDA device ordinal (0) */
     int record_trace;           /* keep the per-iteration line of v2rdm_solver.cc:1881 (0) */
     int profile;                /* time every A / A^T launch of the CG with CUDA events (0) */
-    int adaptive_projection;    /* 1: Update_xz accepts an eigendecomposition whose off-diagonal
-                                   residual is below 0.01 min(eps(p), eps(d)), the CG tolerance
-                                   rule (x, z stay PSD); 0: every projection converged, as the
-                                   plugin (0) */
+    int adaptive_projection;    /* 1: Update_xz accepts a projection whose residual (off-diagonal
+                                   elements of the eigendecomposition, or U (1 - sign^2)) is below
+                                   0.01 min(eps(p), eps(d)), the CG tolerance rule (x, z stay PSD);
+                                   0: every projection converged, as the plugin (0) */
     double cg_tolerance_factor; /* CG stops at factor * min(eps(p), eps(d)) after the first outer
                                    iteration; 0.01 is the plugin's rule (v2rdm_solver.cc:1797-1805),
                                    and values up to 0.1 trade fewer CG iterations for a few more
@@ -99,7 +99,8 @@ typedef struct v2g_options {
                                    3xTF32 products with FP32 accumulation (FP32 accuracy); below it
                                    they run in FP64, whose first refinement sweeps take the
                                    eigenvectors from FP32 to FP64 accuracy.  Maps, CG, errors and
-                                   energies stay FP64.  Needs adaptive_projection (0) */
+                                   energies stay FP64.  Groups small enough to project by the matrix
+                                   sign run it in FP64 throughout.  Needs adaptive_projection (0) */
 } v2g_options;
 
 typedef struct v2g_result {

@@ -67,6 +67,21 @@ def test_small_blocks_match_eigh(v2g, n, positivity, mu):
     _check([d for d in s.dimensions if d > 0], project, 10 * n, mu)
 
 
+@pytest.mark.parametrize("n,positivity", [(9, "DQ"), (7, "DQG"), (10, "DQG"), (13, "DQ"), (16, "D")])
+def test_large_blocks_match_eigh(v2g, n, positivity):
+    # blocks of 81, 98, 100 and 200, 169 and 78, 256 and 120: a team of CTAs each
+    s = v2g.V2RDMSolver([n], (n + 1) // 2, (n + 1) // 2, options=dict(POSITIVITY=positivity))
+    mu = 0.7
+
+    def project(x0):
+        s.set_state(x0, np.zeros(s.nconstraints), np.zeros(s.dimx), mu)
+        s.update_xz(mu)
+        x, _, z, _ = s.get_state()
+        return x, z
+
+    _check([d for d in s.dimensions if d > 0], project, n, mu)
+
+
 def test_small_block_with_a_nan_is_nan(v2g):
     import torch
 

@@ -11,6 +11,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <vector>
 
 namespace v2g {
 
@@ -196,6 +197,27 @@ struct BlockTask {
 void launch_small_project(const BlockTask* tasks, int ntasks, int max_n, int B, const double* aty, const double* c,
                           double* x, double* z, const double* mu, const int* mask, cudaStream_t s,
                           int* hint = nullptr);
+
+// Blocks of any size the same way, a team of CTAs per block in one cooperative
+// launch.  Entry w of a CTA: its w-th block, its rank in the block's team and the
+// team's size (task -1: none).
+struct SignTeam {
+    int task, rank, size;
+    int64_t base;  // of the team's 2 x size partial sums
+};
+// CTAs of the cooperative grid on this device (0: no cooperative launch)
+int sign_grid(int device);
+// Teams of all the blocks on the grid; returns the number of waves (teams: waves
+// x grid entries, a CTA's blocks in its order) and of partial sums.
+int sign_schedule(const std::vector<BlockTask>& tasks, int grid, std::vector<SignTeam>& teams, int64_t& parts);
+// x and z of the blocks of active instances.  atol (per task, optional): accept
+// a residual |U (1 - X^2)|_F of that size.  S, X, X2 and A are np x np workspaces
+// at task.woff; bar one word per task; hint as above; *err = 1 if a team's wait
+// ran out (then the results are invalid).
+cudaError_t launch_team_sign(const BlockTask* tasks, int ntasks, const SignTeam* teams, int waves, int grid, int B,
+                             const double* aty, const double* c, double* x, double* z, const double* mu,
+                             const int* mask, const double* atol, double* S, double* X, double* X2, double* A,
+                             double* part, unsigned int* bar, int* hint, int* err, cudaStream_t s);
 
 // Large blocks (n > 64), block Jacobi on a padded np x np workspace.
 // U = sym(A^T y - c + mu x), zero padded.

@@ -358,7 +358,9 @@ constexpr int kMixedMinNp = 512;
 // Lock-step solve of B instances that share one layout.
 class GroupRun {
   public:
-    GroupRun(DeviceTables& T, std::vector<Problem*> probs) : T_(T), P_(std::move(probs)), B_((int)P_.size()) {
+    // one_shot: for a single projection (v2g_update_xz), not a solve
+    GroupRun(DeviceTables& T, std::vector<Problem*> probs, bool one_shot = false)
+        : T_(T), P_(std::move(probs)), B_((int)P_.size()), one_shot_(one_shot) {
         if (B_ < 1 || B_ > 256) throw std::invalid_argument("a group holds 1..256 instances");
         CK(cudaSetDevice(T.device));
         CK(cudaStreamCreate(&s_));
@@ -393,7 +395,8 @@ class GroupRun {
             ex_.alloc(B_);
         }
         CK(cudaMallocHost(&hscal_, sizeof(double) * 4 * B_));
-        CK(cudaMallocHost(&hnact_, sizeof(int) * 8));
+        CK(cudaMallocHost(&hnact_, sizeof(int) * 9));
+        hnact_[8] = 0;
         CK(cudaMallocHost(&hcs_, sizeof(CgScalars) * B_));
         stage_cap_ = 1 << 20;
         CK(cudaMallocHost(&stage_, stage_cap_));
@@ -496,6 +499,15 @@ class GroupRun {
 
     void project_large(const std::vector<double>& rho) {
         if (nlarge_ == 0) return;
+        if (sign_grid_ > 0) {
+            std::vector<double> at = block_shares(rho);
+            put(atol_.p, at.data(), nlarge_);
+            CK(launch_team_sign(large_d_.p, nlarge_, teams_.p, sign_waves_, sign_grid_, B_, aty_.p, c_.p, x_.p, z_.p,
+                                mu_.p, mask_.p, atol_.p, U_.p, W_.p, Tm_.p, G_.p, signpart_.p, signbar_.p,
+                                sign_hint_.p, signerr_.p, s_));
+            CK(cudaMemcpyAsync(hnact_ + 8, signerr_.p, sizeof(int), cudaMemcpyDeviceToHost, s_));
+            return;
+        }
         launch_form_u(large_d_.p, nlarge_, max_np_, B_, aty_.p, c_.p, x_.p, mu_.p, mask_.p, U_.p, s_);
         set_block_masks();  // bact_ = blocks of active instances
         set_block_tolerances(rho);
@@ -608,6 +620,11 @@ class GroupRun {
             sweeps_total_++;
         }
         launch_lam_from_diag(large_d_.p, nlarge_, W_.p, bjac_.p, lam_.p, s_);
+    }
+
+    // After a synchronisation of the stream.
+    void check_projection() const {
+        if (hnact_[8] != 0) throw CudaError("a team of the projection did not meet (wait ran out)");
     }
 
     cudaStream_t stream() const { return s_; }
@@ -773,6 +790,7 @@ class GroupRun {
             CK(cudaStreamSynchronize(s_));
             stage_synced();
             std::copy(hcs_, hcs_ + B_, cs.begin());
+            check_projection();
             if (tc_ && hnact_[5] != 0)
                 throw CudaError("a tensor-core GEMM of the projection did not finish (pipeline wait ran out)");
             float ms_cg = 0, ms_xz = 0;
@@ -1315,13 +1333,7 @@ class GroupRun {
     // the block; refinement: max |E| <= 1e-7 or residual (~max|E|^2 scale)
     // below the block's rho share.
     void set_block_tolerances(const std::vector<double>& rho) {
-        std::vector<int> nblk(B_, 0);
-        for (int t = 0; t < nlarge_; t++) nblk[hlarge_[t].inst]++;
-        std::vector<double> jt(nlarge_, 1e-13), ot(nlarge_, 1e-7), at(nlarge_, 0.0);
-        for (int t = 0; t < nlarge_; t++) {
-            const int b = hlarge_[t].inst;
-            if (!rho.empty() && rho[b] > 0.0) at[t] = rho[b] / std::sqrt((double)nblk[b]);
-        }
+        std::vector<double> jt(nlarge_, 1e-13), ot(nlarge_, 1e-7), at = block_shares(rho);
         // a fallback block of an instance still far from the solution takes one
         // warm sweep per outer iteration; the next iteration continues from it
         std::vector<int> ms(nlarge_, 1 << 20);
@@ -1339,9 +1351,43 @@ class GroupRun {
         put(atol_.p, at.data(), nlarge_);
     }
 
+    // Each large block's share of its instance's rho (absolute residual it may leave).
+    std::vector<double> block_shares(const std::vector<double>& rho) const {
+        std::vector<int> nblk(B_, 0);
+        for (int t = 0; t < nlarge_; t++) nblk[hlarge_[t].inst]++;
+        std::vector<double> at(nlarge_, 0.0);
+        for (int t = 0; t < nlarge_; t++) {
+            const int b = hlarge_[t].inst;
+            if (!rho.empty() && rho[b] > 0.0) at[t] = rho[b] / std::sqrt((double)nblk[b]);
+        }
+        return at;
+    }
+
     void set_block_masks() {
         // bact[t] = mask[inst(t)], on the device (no round trip through the host)
         launch_block_mask(large_d_.p, nlarge_, mask_.p, bact_.p, s_);
+    }
+
+    // Whether the large blocks take the matrix sign (psd_sign.cu) instead of
+    // kept eigenvectors with refinement.  The sign needs 40 to 70 products a
+    // projection and no host synchronisation, the refinement about 12, but
+    // with a synchronisation per sweep and, where a first-order step is too
+    // large (always in a first projection), Jacobi sweeps; so the sign wins
+    // until the FP64 rate bounds the products.  B200, ms per projection in a
+    // solve, sign / refinement; adaptive projections: n = 10 one instance 0.38
+    // / 0.61, n = 13 four 1.5 / 3.8, n = 20 one 3.2 / 5.7, n = 24 one 8.4 /
+    // 9.4 (2.6e9 = sum of n^3), n = 28 one 20 / 18; many blocks: n = 14 twelve
+    // instances 8.3 / 9.2 (1.2e9), n = 10 a hundred 11.7 / 10.9 (1.3e9).
+    // Exact projections: n = 10 one 0.33 / 3.3, n = 20 one 4.4 / 18.7.
+    bool use_sign() const {
+        const int grid = sign_grid(T_.device);
+        if (grid <= 0) return false;
+        if (one_shot_) return true;
+        double cubes = 0.0;
+        for (const auto& t : hlarge_) cubes += (double)t.n * t.n * t.n;
+        for (auto* p : P_)
+            if (!p->opt.adaptive_projection) return cubes <= 1e10;
+        return cubes <= (2 * nlarge_ <= grid ? 2.6e9 : 1.2e9);
     }
 
     void build_projection_plan() {
@@ -1379,9 +1425,22 @@ class GroupRun {
         if (nlarge_ == 0) return;
         U_.alloc(woff);
         W_.alloc(woff);
-        V_.alloc(woff);
         Tm_.alloc(woff);
         G_.alloc(woff);
+        if (use_sign()) {
+            std::vector<SignTeam> teams;
+            int64_t parts = 0;
+            sign_grid_ = sign_grid(T_.device);
+            sign_waves_ = sign_schedule(hlarge_, sign_grid_, teams, parts);
+            teams_.upload(teams.data(), teams.size());
+            signpart_.alloc(parts);
+            signbar_.alloc(nlarge_);
+            sign_hint_.alloc(nlarge_);
+            signerr_.alloc(1);
+            atol_.alloc(nlarge_);
+            return;
+        }
+        V_.alloc(woff);
         M_.alloc(woff);
         Q_.alloc(qoff);
         qskip_.alloc(qoff / 4096);
@@ -1497,6 +1556,7 @@ class GroupRun {
     DevMap mA_, mAT_;  // the group's copies of the maps, with the tuned kernel variant
     std::vector<Problem*> P_;
     int B_;
+    bool one_shot_;
     int64_t nx_ = 0, nc_ = 0;
     cudaStream_t s_ = nullptr;
     cudaStream_t s_small_ = nullptr;  // the small blocks' projection, beside the large blocks'
@@ -1531,6 +1591,12 @@ class GroupRun {
     DevBuf<unsigned long long> emax_, gdev_;
     DevBuf<int> hard_, bact_, bwork_, bref_, bupd_, bjac_, partner_, msw_, restart_, qskip_;
     DevBuf<double> pthr_;
+    // the matrix sign of the large blocks: grid (0: not used), waves, teams
+    int sign_grid_ = 0, sign_waves_ = 0;
+    DevBuf<SignTeam> teams_;
+    DevBuf<double> signpart_;
+    DevBuf<unsigned int> signbar_;
+    DevBuf<int> sign_hint_, signerr_;
     long restarts_ = 0;
     bool cap_ = false;
     long oa_sweeps_ = 0, jacobi_blocks_ = 0, jacobi_unconverged_ = 0;
@@ -2008,10 +2074,11 @@ int v2g_update_xz(v2g_handle* h, double mu) {
         v2g::require_device();
         Problem& P = h->P;
         P.mu = mu;
-        v2g::GroupRun g(P.tables(), {&P});
+        v2g::GroupRun g(P.tables(), {&P}, true);
         g.project();
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(g.stream()));
+        g.check_projection();
         g.download_state();
         return V2G_OK;
     });
