@@ -8,17 +8,20 @@
 
 namespace v2g {
 
-// C[M x N] = op(A)[M x K] op(B)[K x N] (+ bias) (ReLU) (C += when accumulate),
-// row-major with leading dimensions; FP32 arithmetic, deterministic.
-void mlp_gemm(int M, int N, int K, const float* A, int lda, bool transA, const float* B, int ldb, bool transB,
-              const float* bias, bool relu, bool accumulate, float* C, int ldc, cudaStream_t s);
-// the same with BF16 B (the weights)
-void mlp_gemm_bf16(int M, int N, int K, const float* A, int lda, bool transA, const __nv_bfloat16* B, int ldb,
-                   bool transB, const float* bias, bool relu, bool accumulate, float* C, int ldc, cudaStream_t s);
-// dy[i] = 0 where y[i] <= 0
-void mlp_relu_back(int64_t n, const float* y, float* dy, cudaStream_t s);
-// db[n] = sum over rows of dy[m, n]
-void mlp_col_sum(int M, int N, const float* dy, float* db, cudaStream_t s);
+// A layer: C[M x N] = A[M x K] W^T + bias (ReLU), W (N x K) in BF16; FP32
+// arithmetic, deterministic, like everything here.
+void mlp_layer(int M, int N, int K, const float* A, const __nv_bfloat16* W, const float* bias, bool relu, float* C,
+               cudaStream_t s);
+// dx[M x N] = dy[M x K] W (W: K x N), zero where gate <= 0 (the ReLU of the layer below)
+void mlp_input_grad(int M, int N, int K, const float* dy, const __nv_bfloat16* W, const float* gate, float* dx,
+                    cudaStream_t s);
+// Slice k of mlp_slices(rows): its partial dW (out x in) = dy^T x at dw + k * stride,
+// its partial db (column sums of dy) at db + k * stride
+int mlp_slices(int rows);
+void mlp_weight_grad(int rows, int out, int in, const float* dy, const float* x, float* dw, float* db, int64_t stride,
+                     cudaStream_t s);
+// g[i] = sum over slices of part[k * n + i]
+void mlp_sum_slices(int64_t n, int slices, const float* part, float* g, cudaStream_t s);
 // d = 2 (out - t) scale; partial[block] = sum (out - t)^2 (mlp_mse_blocks() blocks)
 int mlp_mse_blocks();
 void mlp_mse(int64_t n, const float* out, const float* t, float scale, float* d, double* partial, cudaStream_t s);

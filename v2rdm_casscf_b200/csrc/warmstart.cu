@@ -67,7 +67,7 @@ struct WsNet {
     Buf<float> w, m, v, g;
     Buf<__nv_bfloat16> w16;
     // activations of the last forward pass: act[0] = input rows, act[l + 1] = layer l's output
-    Buf<float> act[kWsLayers + 1], dact[2], targ, delta;
+    Buf<float> act[kWsLayers + 1], dact[2], targ, delta, gpart;
     Buf<double> partial;
     int64_t rows_cap = 0;
     int step = 0;
@@ -118,13 +118,14 @@ struct WsNet {
         targ.ensure((size_t)rows * kWsOut);
         delta.ensure((size_t)rows * kWsOut);
         partial.ensure(mlp_mse_blocks());
+        if (mlp_slices((int)rows) > 1) gpart.ensure((size_t)mlp_slices((int)rows) * nparams);
         rows_cap = rows;
     }
     // act[kWsLayers] = network(act[0]) for `rows` rows
     void forward(int rows) {
         for (int l = 0; l < kWsLayers; l++)
-            mlp_gemm_bf16(rows, dims[l + 1], dims[l], act[l].p, dims[l], false, w16.p + woff[l], dims[l], true,
-                          w.p + boff[l], l + 1 < kWsLayers, false, act[l + 1].p, dims[l + 1], s);
+            mlp_layer(rows, dims[l + 1], dims[l], act[l].p, w16.p + woff[l], w.p + boff[l], l + 1 < kWsLayers,
+                      act[l + 1].p, s);
     }
     // g = d(mean squared error)/d(params) for the last forward pass against
     // targ; returns the loss (mean over rows and outputs)
@@ -133,20 +134,21 @@ struct WsNet {
         mlp_mse(nout, act[kWsLayers].p, targ.p, 1.f / (float)nout, delta.p, partial.p, s);
         const float* dy = delta.p;
         int cur = 0;
+        // the slices' partial gradients (one slice: the gradient itself)
+        const int slices = mlp_slices(rows);
+        float* part = slices > 1 ? gpart.p : g.p;
         for (int l = kWsLayers - 1; l >= 0; l--) {
             const int out = dims[l + 1], in = dims[l];
-            // dW_l = dY^T act_l (out x in), db_l = column sums of dY
-            mlp_gemm(out, in, rows, dy, out, true, act[l].p, in, false, nullptr, false, false, g.p + woff[l], in, s);
-            mlp_col_sum(rows, out, dy, g.p + boff[l], s);
+            // dW_l = dY^T act_l (out x in), db_l = column sums of dY, per slice
+            mlp_weight_grad(rows, out, in, dy, act[l].p, part + woff[l], part + boff[l], nparams, s);
             if (l == 0) break;
-            // dX = dY W_l, then through the ReLU of layer l - 1
+            // dX = dY W_l, through the ReLU of layer l - 1
             float* dx = dact[cur].p;
-            mlp_gemm_bf16(rows, in, out, dy, out, false, w16.p + woff[l], in, false, nullptr, false, false, dx, in,
-                          s);
-            mlp_relu_back((int64_t)rows * in, act[l].p, dx, s);
+            mlp_input_grad(rows, in, out, dy, w16.p + woff[l], act[l].p, dx, s);
             dy = dx;
             cur ^= 1;
         }
+        if (slices > 1) mlp_sum_slices(nparams, slices, part, g.p, s);
         std::vector<double> hp(mlp_mse_blocks());
         WCK(cudaMemcpyAsync(hp.data(), partial.p, hp.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
         WCK(cudaStreamSynchronize(s));
