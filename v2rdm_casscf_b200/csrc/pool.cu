@@ -1,0 +1,107 @@
+#include "pool.h"
+
+#include <map>
+#include <mutex>
+#include <vector>
+
+namespace v2g {
+
+namespace {
+
+std::mutex g_mu;
+// per device: the pool, or nullptr where the device has no stream-ordered allocator
+std::map<int, cudaMemPool_t> g_pools;
+std::multimap<size_t, void*> g_pinned;
+size_t g_pinned_bytes = 0;
+
+cudaMemPool_t pool_of(int device) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_pools.find(device);
+    if (it != g_pools.end()) return it->second;
+    cudaMemPool_t pool = nullptr;
+    int ok = 0;
+    if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, device) == cudaSuccess && ok) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        unsigned long long keep = kPoolKeep;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+            pool = nullptr;
+        } else if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            pool = nullptr;
+        }
+        if (!pool) cudaGetLastError();
+    }
+    return g_pools[device] = pool;
+}
+
+size_t pinned_size(size_t bytes) {
+    size_t s = 4096;
+    while (s < bytes) s *= 2;
+    return s;
+}
+
+}  // namespace
+
+cudaError_t pool_alloc(void** p, size_t bytes) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    const cudaMemPool_t pool = pool_of(device);
+    if (!pool) return cudaMalloc(p, bytes);
+    e = cudaMallocFromPoolAsync(p, bytes, pool, cudaStreamLegacy);
+    if (e == cudaErrorMemoryAllocation) {
+        // what the pool holds unused may be in the way
+        cudaGetLastError();
+        cudaStreamSynchronize(cudaStreamLegacy);
+        cudaMemPoolTrimTo(pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, cudaStreamLegacy);
+    }
+    return e;
+}
+
+void pool_free(void* p, int device) {
+    if (!p) return;
+    int prev = -1;
+    if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
+    if (prev != device) cudaSetDevice(device);
+    if (pool_of(device))
+        cudaFreeAsync(p, cudaStreamLegacy);
+    else
+        cudaFree(p);
+    if (prev >= 0 && prev != device) cudaSetDevice(prev);
+}
+
+cudaError_t pinned_alloc(void** p, size_t bytes) {
+    const size_t size = pinned_size(bytes);
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        auto it = g_pinned.find(size);
+        if (it != g_pinned.end()) {
+            *p = it->second;
+            g_pinned.erase(it);
+            g_pinned_bytes -= size;
+            return cudaSuccess;
+        }
+    }
+    return cudaMallocHost(p, size);
+}
+
+void pinned_free(void* p, size_t bytes) {
+    if (!p) return;
+    const size_t size = pinned_size(bytes);
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (g_pinned_bytes + size <= kPinnedKeep) {
+            g_pinned.emplace(size, p);
+            g_pinned_bytes += size;
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+}  // namespace v2g

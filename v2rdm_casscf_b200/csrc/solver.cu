@@ -30,6 +30,7 @@
 #include "constraints.h"
 #include "kernels.cuh"
 #include "layout.h"
+#include "pool.h"
 #include "warmstart.h"
 
 namespace v2g {
@@ -72,25 +73,48 @@ template <class T>
 struct DevBuf {
     T* p = nullptr;
     size_t n = 0;
+    int device = 0;
     DevBuf() = default;
     explicit DevBuf(size_t count) { alloc(count); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    ~DevBuf() {
-        if (p) cudaFree(p);
-    }
-    void alloc(size_t count) {
-        if (p) cudaFree(p);
+    ~DevBuf() { pool_free(p, device); }
+    // zeroed unless every element is written before it is read
+    void alloc(size_t count, bool zero = true) {
+        pool_free(p, device);
         p = nullptr;
         n = count;
         if (count) {
-            CK(cudaMalloc(&p, count * sizeof(T)));
-            CK(cudaMemset(p, 0, count * sizeof(T)));
+            CK(cudaGetDevice(&device));
+            void* q = nullptr;
+            CK(pool_alloc(&q, count * sizeof(T)));
+            p = static_cast<T*>(q);
+            if (zero) CK(cudaMemsetAsync(p, 0, count * sizeof(T), cudaStreamLegacy));
         }
     }
     void upload(const T* h, size_t count) {
-        alloc(count);
+        alloc(count, false);
         if (count) CK(cudaMemcpy(p, h, count * sizeof(T), cudaMemcpyHostToDevice));
+    }
+};
+
+// Page-locked host memory for copies on the streams of its owner.
+template <class T>
+struct HostBuf {
+    T* p = nullptr;
+    size_t n = 0;
+    HostBuf() = default;
+    HostBuf(const HostBuf&) = delete;
+    HostBuf& operator=(const HostBuf&) = delete;
+    ~HostBuf() { pinned_free(p, n * sizeof(T)); }
+    void alloc(size_t count) {
+        pinned_free(p, n * sizeof(T));
+        p = nullptr;
+        n = 0;
+        void* q = nullptr;
+        CK(pinned_alloc(&q, count * sizeof(T)));
+        p = static_cast<T*>(q);
+        n = count;
     }
 };
 
@@ -370,40 +394,43 @@ class GroupRun {
         nx_ = T.L.dimx;
         nc_ = T.L.ncon;
         const size_t X = (size_t)nx_ * B_, C = (size_t)nc_ * B_;
-        c_.alloc(X);
-        x_.alloc(X);
-        z_.alloc(X);
+        c_.alloc(X, false);
+        x_.alloc(X, false);
+        z_.alloc(X, false);
+        y_.alloc(C, false);
         aty_.alloc(X);
+        mu_.alloc(B_);
+        mask_.alloc(B_);
+        nact_.alloc(8);  // counters: CG, Jacobi, refinement, fallback, restart
+        hnact_buf_.alloc(9);
+        hnact_ = hnact_buf_.p;
+        hnact_[8] = 0;
+        stage_.alloc(one_shot_ ? 1 << 16 : 1 << 20);
+        mA_ = T.A();
+        mAT_ = T.AT();
+        build_projection_plan();
+        upload_state();
+        if (one_shot_) return;
         atp_.alloc(X);
-        y_.alloc(C);
         ax_.alloc(C);
         bv_.alloc(C);
         r_.alloc(C);
         p_.alloc(C);
         partial_.alloc(reduce_partial_size(B_) + (int64_t)(T.max_long() + 8) * B_);
         red_.alloc(4 * B_);
-        mu_.alloc(B_);
         coef_.alloc(B_);
-        mask_.alloc(B_);
         smask1_.alloc(B_);
         smask2_.alloc(B_);
         cs_.alloc(B_);
-        nact_.alloc(8);  // counters: CG, Jacobi, refinement, fallback, restart
         for (auto* p : P_) extrapolate_ = extrapolate_ || p->opt.cg_extrapolate;
         if (extrapolate_) {
             yprev_.alloc(C);
             ex_.alloc(B_);
         }
-        CK(cudaMallocHost(&hscal_, sizeof(double) * 4 * B_));
-        CK(cudaMallocHost(&hnact_, sizeof(int) * 9));
-        hnact_[8] = 0;
-        CK(cudaMallocHost(&hcs_, sizeof(CgScalars) * B_));
-        stage_cap_ = 1 << 20;
-        CK(cudaMallocHost(&stage_, stage_cap_));
-        mA_ = T.A();
-        mAT_ = T.AT();
-        build_projection_plan();
-        upload_state();
+        hscal_buf_.alloc(4 * B_);
+        hscal_ = hscal_buf_.p;
+        hcs_buf_.alloc(B_);
+        hcs_ = hcs_buf_.p;
         tune_maps();
         if (cg_loop_fits(nc_, B_)) loop_grid_ = cg_loop_grid(T.device);
         if (loop_grid_ > 0) {
@@ -421,15 +448,13 @@ class GroupRun {
         }
     }
     ~GroupRun() {
+        // nothing may still be in flight on the buffers that go back to the pools
+        if (s_) cudaStreamSynchronize(s_);
+        if (s_small_) cudaStreamSynchronize(s_small_);
         if (cg_exec_) cudaGraphExecDestroy(cg_exec_);
         if (cg_loop_exec_) cudaGraphExecDestroy(cg_loop_exec_);
         if (diag_file_) std::fclose(diag_file_);
         for (auto e : prof_ev_) cudaEventDestroy(e);
-        if (hscal_) cudaFreeHost(hscal_);
-        if (hnact_) cudaFreeHost(hnact_);
-        if (hcs_) cudaFreeHost(hcs_);
-        if (hdots_ptr_) cudaFreeHost(hdots_ptr_);
-        if (stage_) cudaFreeHost(stage_);
         if (ev_fork_) cudaEventDestroy(ev_fork_);
         if (ev_join_) cudaEventDestroy(ev_join_);
         if (s_small_) cudaStreamDestroy(s_small_);
@@ -438,6 +463,10 @@ class GroupRun {
 
     // Interleave host vectors of all instances into [e * B + b].
     void upload_vec(DevBuf<double>& d, int64_t n, const std::vector<double> Problem::*member) {
+        if (B_ == 1) {
+            CK(cudaMemcpy(d.p, (P_[0]->*member).data(), n * sizeof(double), cudaMemcpyHostToDevice));
+            return;
+        }
         std::vector<double> h((size_t)n * B_);
         for (int b = 0; b < B_; b++) {
             const auto& v = P_[b]->*member;
@@ -446,6 +475,11 @@ class GroupRun {
         CK(cudaMemcpy(d.p, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
     void download_vec(const DevBuf<double>& d, int64_t n, std::vector<double> Problem::*member) {
+        if (B_ == 1) {
+            (P_[0]->*member).resize(n);
+            CK(cudaMemcpy((P_[0]->*member).data(), d.p, n * sizeof(double), cudaMemcpyDeviceToHost));
+            return;
+        }
         std::vector<double> h((size_t)n * B_);
         CK(cudaMemcpy(h.data(), d.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost));
         for (int b = 0; b < B_; b++) {
@@ -468,7 +502,7 @@ class GroupRun {
     void download_state() {
         download_vec(x_, nx_, &Problem::x);
         download_vec(z_, nx_, &Problem::z);
-        download_vec(y_, nc_, &Problem::y);
+        if (!one_shot_) download_vec(y_, nc_, &Problem::y);
     }
 
     // Update_xz for every instance with mask set; ATy is left in aty_.
@@ -928,16 +962,11 @@ class GroupRun {
         launch_aa_update(nx_, B_, aa_m_, x_.p, z_.p, aw_.p, af_.p, ag_.p, adF_.p, adG_.p, amode_.p, aslot_.p,
                          apart_.p, adots_.p, s_);
         const size_t ndots = (size_t)(2 * aa_m_ + 1) * B_;
-        if (hdots_.size() < ndots) {
-            if (hdots_ptr_) CK(cudaFreeHost(hdots_ptr_));
-            hdots_ptr_ = nullptr;
-            CK(cudaMallocHost(&hdots_ptr_, ndots * sizeof(double)));
-            hdots_.assign(ndots, 0.0);
-        }
-        CK(cudaMemcpyAsync(hdots_ptr_, adots_.p, ndots * sizeof(double), cudaMemcpyDeviceToHost, s_));
+        if (hdots_.n < ndots) hdots_.alloc(ndots);
+        CK(cudaMemcpyAsync(hdots_.p, adots_.p, ndots * sizeof(double), cudaMemcpyDeviceToHost, s_));
         CK(cudaStreamSynchronize(s_));
         stage_synced();
-        std::vector<double> dots(hdots_ptr_, hdots_ptr_ + ndots);
+        std::vector<double> dots(hdots_.p, hdots_.p + ndots);
         std::vector<double> gamma((size_t)B_ * aa_m_, 0.0);
         std::vector<int> mix(B_, 0);
         bool anymix = false;
@@ -1134,18 +1163,13 @@ class GroupRun {
         const size_t bytes = n * sizeof(T);
         if (bytes == 0) return;
         size_t off = (stage_off_ + 15) & ~(size_t)15;
-        if (off + bytes > stage_cap_) {
+        if (off + bytes > stage_.n) {
             CK(cudaStreamSynchronize(s_));
             off = 0;
-            if (bytes > stage_cap_) {
-                CK(cudaFreeHost(stage_));
-                stage_ = nullptr;
-                stage_cap_ = bytes;
-                CK(cudaMallocHost(&stage_, stage_cap_));
-            }
+            if (bytes > stage_.n) stage_.alloc(bytes);
         }
-        std::memcpy(stage_ + off, src, bytes);
-        CK(cudaMemcpyAsync(dst, stage_ + off, bytes, cudaMemcpyHostToDevice, s_));
+        std::memcpy(stage_.p + off, src, bytes);
+        CK(cudaMemcpyAsync(dst, stage_.p + off, bytes, cudaMemcpyHostToDevice, s_));
         stage_off_ = off + bytes;
     }
     void stage_synced() { stage_off_ = 0; }
@@ -1423,11 +1447,12 @@ class GroupRun {
         small_hint_.alloc(small.size());
         large_d_.upload(hlarge_.data(), hlarge_.size());
         if (nlarge_ == 0) return;
-        U_.alloc(woff);
-        W_.alloc(woff);
-        Tm_.alloc(woff);
-        G_.alloc(woff);
-        if (use_sign()) {
+        const bool sign = use_sign();
+        U_.alloc(woff, !sign);
+        W_.alloc(woff, !sign);
+        Tm_.alloc(woff, !sign);
+        G_.alloc(woff, !sign);
+        if (sign) {
             std::vector<SignTeam> teams;
             int64_t parts = 0;
             sign_grid_ = sign_grid(T_.device);
@@ -1578,11 +1603,12 @@ class GroupRun {
     DevBuf<int> amode_, aslot_, amix_;
     double* hscal_ = nullptr;
     int* hnact_ = nullptr;
-    char* stage_ = nullptr;
-    size_t stage_cap_ = 0, stage_off_ = 0;
+    HostBuf<double> hscal_buf_, hdots_;
+    HostBuf<int> hnact_buf_;
+    HostBuf<CgScalars> hcs_buf_;
+    HostBuf<char> stage_;
+    size_t stage_off_ = 0;
     CgScalars* hcs_ = nullptr;  // pinned copy of the CG scalars after a CG solve
-    double* hdots_ptr_ = nullptr;  // pinned Anderson dot products
-    std::vector<double> hdots_;
     // projection plan
     std::vector<BlockTask> hlarge_;
     DevBuf<BlockTask> small_d_, large_d_;
@@ -2346,6 +2372,7 @@ int v2g_time_maps(v2g_handle* h, int nvec, int reps, double* sec_A, double* sec_
         const int64_t nx = T.L.dimx, nc = T.L.ncon;
         v2g::DevBuf<double> x((size_t)nx * nvec), y((size_t)nc * nvec), ox((size_t)nx * nvec), oy((size_t)nc * nvec);
         cudaStream_t s = nullptr;
+        CK(cudaStreamSynchronize(cudaStreamLegacy));  // the buffers are ready for a non-blocking stream
         CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         cudaGraphExec_t ex = nullptr;
@@ -2353,7 +2380,10 @@ int v2g_time_maps(v2g_handle* h, int nvec, int reps, double* sec_A, double* sec_
             if (ex) cudaGraphExecDestroy(ex);
             if (e0) cudaEventDestroy(e0);
             if (e1) cudaEventDestroy(e1);
-            if (s) cudaStreamDestroy(s);
+            if (s) {
+                cudaStreamSynchronize(s);
+                cudaStreamDestroy(s);
+            }
         };
         try {
             CK(cudaEventCreate(&e0));
@@ -2447,8 +2477,9 @@ struct BlockGemmPlan {
         dg.upload(tiles.data(), tiles.size());
         if (use_tc) {
             ds.upload(split.data(), split.size());
-            wa.alloc(toff);
-            wb.alloc(toff);
+            // the split writes every word of its tiles
+            wa.alloc(toff, false);
+            wb.alloc(toff, false);
             tc.tasks = dt.p;
             tc.tiles_full = dg.p;
             tc.n_full = (int)tiles.size();
@@ -2500,12 +2531,16 @@ int v2g_time_block_gemm(int nblocks, const int* dims, const double* A, const dou
         if (!plan.build(nblocks, dims, tensor_cores != 0))
             return v2g::fail(V2G_ERR_ARG, "block dimension out of range");
         cudaStream_t s = nullptr;
+        CK(cudaStreamSynchronize(cudaStreamLegacy));  // the buffers are ready for a non-blocking stream
         CK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         auto cleanup = [&]() {
             if (e0) cudaEventDestroy(e0);
             if (e1) cudaEventDestroy(e1);
-            if (s) cudaStreamDestroy(s);
+            if (s) {
+                cudaStreamSynchronize(s);
+                cudaStreamDestroy(s);
+            }
         };
         try {
             CK(cudaEventCreate(&e0));
