@@ -76,21 +76,23 @@ constexpr int kMapVariants = 2;  // 0: plain, 1: streamed
 void launch_spmv(const DevMap& A, int B, const double* in, double* out, const double* sub, const double* coef,
                  const double* add, const int* mask, cudaStream_t s);
 
-// Per-instance reductions over interleaved vectors of n elements.
-enum ReduceMode {
-    RED_DOT = 0,      // sum u*v
-    RED_ED = 1,       // sum ((u + v) - w)^2       (dual error, v2rdm_solver.cc:1829-1832)
-    RED_EP = 2,       // sum (u - row[e])^2        (primal error, v2rdm_solver.cc:1835-1837)
-    RED_DOT_ROW = 3,  // sum u * row[e]            (b . y)
-};
-// Writes one value per instance to out[0..B).  partial must hold
-// reduce_partial_size(B) doubles.  Deterministic summation order.
-void launch_reduce(ReduceMode mode, int64_t n, int B, const double* u, const double* v, const double* w,
-                   const double* row, double* partial, double* out, cudaStream_t s);
+// out[b] = u . v per instance over interleaved vectors of n elements
+// (deterministic).  partial holds reduce_partial_size(B) doubles.
+void launch_dot(int64_t n, int B, const double* u, const double* v, double* partial, double* out, cudaStream_t s);
 int64_t reduce_partial_size(int B);
 
-// z = c - z for active instances (v2rdm_solver.cc:1789-1790)
-void launch_c_minus_z(int64_t n, int B, const double* c, double* z, const int* mask, cudaStream_t s);
+// The right-hand side of the dual step (v2rdm_solver.cc:1783-1794) for the
+// instances of mask: z <- c - z + coef x with coef = -tau mu, rhs = A z - coef b.
+// The reference forms A (c - z) and -tau mu (A x - b) apart; one map does both.
+// With w (2 nx rows), w <- (x, z) before, where mode[b] != 0.
+void launch_rhs(const DevMap& A, int64_t nx, int B, const double* c, const double* x, double* z, const double* brow,
+                const double* coef, const int* mask, double* w, const int* mode, double* rhs, cudaStream_t s);
+
+// red[0..B) = |A^T y + z - c|^2, red[B..) = |A x - b|^2, red[2 B..) = c . x,
+// red[3 B..) = b . y (v2rdm_solver.cc:1826-1852), deterministic.
+void launch_errors(const DevMap& A, int64_t nx, int64_t nc, int B, const double* aty, const double* x, const double* y,
+                   const double* z, const double* c, const double* brow, const int* mask, double* partial, double* red,
+                   cudaStream_t s);
 // out[e * B + b] = row[e] (or 0 when row is null) for the instances with mask[b] set
 void launch_set_rows(int64_t n, int B, const double* row, double* out, const int* mask, cudaStream_t s);
 
@@ -161,8 +163,6 @@ void launch_cg_extrapolate(int64_t n, int B, double* y, double* yprev, const int
 // g = the iterate the step produced), each 2 * nx * B doubles, column j at
 // j * 2 * nx * B.
 constexpr int kAndersonMax = 16;
-// w <- (x, z) for the instances with mode[b] != 0
-void launch_aa_save(int64_t nx, int B, const double* x, const double* z, double* w, const int* mode, cudaStream_t s);
 // f = g - w; mode[b] == 2: dF[slot[b]] = f - fprev, dG[slot[b]] = g - gprev and
 // dots[(2 j) * B + b] = dF[slot].dF[j], dots[(2 j + 1) * B + b] = dF[j].f for j < m;
 // mode[b] >= 1: dots[(2 m) * B + b] = f.f, fprev = f, gprev = g.  partial holds
@@ -194,9 +194,10 @@ struct BlockTask {
 // Blocks with n <= 64 (max_n the largest of them): form U, its matrix sign in
 // shared memory, x and z (psd_sign.cu).  hint (optional, one word per task, 0 at
 // first) carries the number of lift steps that sufficed to the next call.
+// beside: the launch shares the GPU with launch_team_sign.
 void launch_small_project(const BlockTask* tasks, int ntasks, int max_n, int B, const double* aty, const double* c,
                           double* x, double* z, const double* mu, const int* mask, cudaStream_t s,
-                          int* hint = nullptr);
+                          int* hint = nullptr, bool beside = false);
 
 // Blocks of any size the same way, a team of CTAs per block in one cooperative
 // launch.  Entry w of a CTA: its w-th block, its rank in the block's team and the

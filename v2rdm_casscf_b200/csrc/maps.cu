@@ -269,6 +269,44 @@ struct EpiAffine {
     }
 };
 
+// out = A in - coef brow: the right-hand side A (c - z - tau mu x) + tau mu b
+// of the dual step with coef = -tau mu
+struct EpiRhs {
+    static constexpr bool kSum = false;
+    const double* brow;
+    const double* coef;
+    double* out;
+    const int* mask;
+    using Own = OwnNone;
+    template <bool COH>
+    __device__ __forceinline__ Own own(int32_t, int, int) const {
+        return {};
+    }
+    __device__ __forceinline__ bool on(int b) const { return !mask || mask[b]; }
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t r, int B, int b, double s, const Own&) const {
+        out[(int64_t)r * B + b] = s - coef[b] * brow[r];
+        return 0.0;
+    }
+};
+// sums |A in - brow|^2, stores nothing
+struct EpiResidual {
+    static constexpr bool kSum = true;
+    const double* brow;
+    const int* mask;
+    using Own = OwnNone;
+    template <bool COH>
+    __device__ __forceinline__ Own own(int32_t, int, int) const {
+        return {};
+    }
+    __device__ __forceinline__ bool on(int b) const { return !mask || mask[b]; }
+    template <bool COH>
+    __device__ __forceinline__ double one(int32_t r, int B, int b, double s, const Own&) const {
+        const double d = s - brow[r];
+        return d * d;
+    }
+};
+
 // The CG iteration (cg_solver.cc:141-177) in two map applications, every
 // vector update in the epilogue of the map that produces its input:
 //   q = A^T r + beta q   (= A^T p for the new p = r + beta p), summing q.q = p.A A^T p
@@ -617,10 +655,9 @@ __global__ void __launch_bounds__(kThreads, kMapCtasPerSm)
     if (Epi::kSum && (int)threadIdx.x < B) partial[(int64_t)blockIdx.x * B + threadIdx.x] = s;
 }
 
-// Stage 1: block g reduces a contiguous chunk of elements for every instance;
-// thread t handles instance t % B on element rows t / B, t / B + T/B, ...
-__global__ void reduce_stage1(int mode, int64_t n, int B, const double* __restrict__ u, const double* __restrict__ v,
-                              const double* __restrict__ w, const double* __restrict__ row,
+// Stage 1: block g reduces a contiguous chunk of elements of u . v for every
+// instance; thread t handles instance t % B on element rows t / B, t / B + T/B, ...
+__global__ void reduce_stage1(int64_t n, int B, const double* __restrict__ u, const double* __restrict__ v,
                               double* __restrict__ partial) {
     const int rows_per_pass = blockDim.x / B;
     const int lanes = rows_per_pass * B;
@@ -631,28 +668,59 @@ __global__ void reduce_stage1(int mode, int64_t n, int B, const double* __restri
         const int64_t chunk = (n + gridDim.x - 1) / gridDim.x;
         const int64_t e0 = blockIdx.x * chunk;
         const int64_t e1 = (e0 + chunk < n) ? e0 + chunk : n;
-        for (int64_t e = e0 + rsub; e < e1; e += rows_per_pass) {
-            const int64_t i = e * B + b;
-            double term;
-            switch (mode) {
-                case RED_DOT: term = u[i] * v[i]; break;
-                case RED_ED: {
-                    double d = (u[i] + v[i]) - w[i];
-                    term = d * d;
-                    break;
-                }
-                case RED_EP: {
-                    double d = u[i] - row[e];
-                    term = d * d;
-                    break;
-                }
-                default: term = u[i] * row[e]; break;
-            }
-            acc += term;
-        }
+        for (int64_t e = e0 + rsub; e < e1; e += rows_per_pass) acc += u[e * B + b] * v[e * B + b];
     }
     const double s = cta_instance_sum(acc, B);
     if ((int)threadIdx.x < B) partial[(int64_t)blockIdx.x * B + threadIdx.x] = s;
+}
+
+// The outer iteration's sums over the primal and dual vectors in one pass, with
+// the residual map and one final kernel for all four (nine launches before; n = 5
+// on a B200: 72 -> 49 us per outer iteration outside CG and projection, with the
+// right-hand side in one map instead of two)
+// (v2rdm_solver.cc:1826-1852): partial[k * gridDim.x * B + block * B + b] for
+// k = 0 |A^T y + z - c|^2, 1 c . x, 2 b . y.
+__global__ void __launch_bounds__(kThreads) sums_kernel(int64_t nx, int64_t nc, int B, const double* __restrict__ aty,
+                                                        const double* __restrict__ z, const double* __restrict__ c,
+                                                        const double* __restrict__ x, const double* __restrict__ y,
+                                                        const double* __restrict__ brow, double* __restrict__ partial) {
+    double ed = 0.0, cx = 0.0, by = 0.0;
+    const Chunk px = chunk_of(nx, B), py = chunk_of(nc, B);
+    if (px.live) {
+        for (int64_t e = px.first; e < nx; e += px.stride) {
+            const int64_t i = e * B + px.b;
+            const double cv = c[i], d = (aty[i] + z[i]) - cv;
+            ed += d * d;
+            cx += cv * x[i];
+        }
+        for (int64_t e = py.first; e < nc; e += py.stride) by += y[e * B + py.b] * brow[e];
+    }
+    const double v[3] = {ed, cx, by};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const double s = cta_instance_sum(v[k], B);
+        if ((int)threadIdx.x < B) partial[((int64_t)k * gridDim.x + blockIdx.x) * B + threadIdx.x] = s;
+    }
+}
+
+// red[k * B + b] from the partials of sums_kernel (nsums blocks) and of the
+// residual map (nres blocks, after them): ed^2, ep^2, c . x, b . y; one CTA each.
+__global__ void errors_kernel(int nsums, int nres, int B, const double* __restrict__ partial,
+                              double* __restrict__ red) {
+    __shared__ double sh[kThreads];
+    const int k = blockIdx.x / B, b = blockIdx.x % B;
+    const int part = k == 0 ? 0 : (k == 1 ? 3 : k - 1);
+    const int n = k == 1 ? nres : nsums;
+    const double* p = partial + (int64_t)part * nsums * B;
+    double s = 0.0;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s += p[(int64_t)i * B + b];
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+        if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) red[blockIdx.x] = sh[0];
 }
 
 // Stage 2: one block per instance sums its nblk partials with a fixed tree
@@ -683,14 +751,23 @@ __global__ void set_rows_kernel(int64_t n, int B, const double* __restrict__ row
     }
 }
 
-__global__ void c_minus_z_kernel(int64_t n, int B, const double* __restrict__ c, double* __restrict__ z,
-                                 const int* __restrict__ mask) {
+// z <- c - z + coef x (coef = -tau mu): the input of the right-hand side's map;
+// with w, w <- (x, z) first for the instances with mode[b] != 0 (the state the
+// Anderson step starts from)
+__global__ void rhs_input_kernel(int64_t n, int B, const double* __restrict__ c, const double* __restrict__ x,
+                                 double* __restrict__ z, const double* __restrict__ coef, const int* __restrict__ mask,
+                                 double* __restrict__ w, const int* __restrict__ mode) {
     const int64_t total = n * B;
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
          t += (int64_t)gridDim.x * blockDim.x) {
         const int b = (int)(t % B);
-        if (mask && !mask[b]) continue;
-        z[t] = -z[t] + c[t];
+        if (!mask[b]) continue;
+        const double xv = x[t], zv = z[t];
+        if (w && mode[b]) {
+            w[t] = xv;
+            w[total + t] = zv;
+        }
+        z[t] = (c[t] - zv) + coef[b] * xv;
     }
 }
 
@@ -708,16 +785,6 @@ __global__ void cg_extrapolate_kernel(int64_t n, int B, double* __restrict__ y, 
 }
 
 // ---- Anderson acceleration (kernels.cuh) ----
-
-__global__ void aa_save_kernel(int64_t nx, int B, const double* __restrict__ x, const double* __restrict__ z,
-                               double* __restrict__ w, const int* __restrict__ mode) {
-    const int64_t half = nx * B, total = 2 * half;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        if (!mode[(int)(t % B)]) continue;
-        w[t] = (t < half) ? x[t] : z[t - half];
-    }
-}
 
 // Rows e of the state are walked with the chunk mapping of the reducing
 // kernels, so each thread keeps one instance and its 2 m dot products come
@@ -1216,14 +1283,6 @@ __global__ void __launch_bounds__(ONE ? kResThreads : 768, 1) cg_resident_kernel
 
 }  // namespace
 
-static int spmv_grid(int64_t nrows, int B) {
-    // enough blocks to fill the GPU; rows per block >= rows per pass
-    const int64_t rows_per_pass = kThreads / B;
-    int64_t g = (nrows + rows_per_pass - 1) / rows_per_pass;
-    if (g > kSpmvBlocks) g = kSpmvBlocks;
-    return (int)(g < 1 ? 1 : g);
-}
-
 // Whether table loads and output stores bypass the caches (streaming hints):
 // the autotuner's choice, or streamed from eight instances up.
 static bool map_streamed(const DevMap& M, int B) {
@@ -1300,11 +1359,29 @@ void launch_spmv(const DevMap& A, int B, const double* in, double* out, const do
 
 int64_t reduce_partial_size(int B) { return (int64_t)kSpmvBlocks * B; }
 
-void launch_reduce(ReduceMode mode, int64_t n, int B, const double* u, const double* v, const double* w,
-                   const double* row, double* partial, double* out, cudaStream_t s) {
-    reduce_stage1<<<kRedBlocks, kThreads, 0, s>>>((int)mode, n, B, u, v, w, row, partial);
+void launch_dot(int64_t n, int B, const double* u, const double* v, double* partial, double* out, cudaStream_t s) {
+    reduce_stage1<<<kRedBlocks, kThreads, 0, s>>>(n, B, u, v, partial);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
     reduce_stage2<<<B, kThreads, 0, s>>>(kRedBlocks, B, partial, out);
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+}
+
+void launch_rhs(const DevMap& A, int64_t nx, int B, const double* c, const double* x, double* z, const double* brow,
+                const double* coef, const int* mask, double* w, const int* mode, double* rhs, cudaStream_t s) {
+    rhs_input_kernel<<<grid_for(nx * B), kThreads, 0, s>>>(nx, B, c, x, z, coef, mask, w, mode);
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    run_map(A, B, z, EpiRhs{brow, coef, rhs, mask}, nullptr, s);
+}
+
+void launch_errors(const DevMap& A, int64_t nx, int64_t nc, int B, const double* aty, const double* x, const double* y,
+                   const double* z, const double* c, const double* brow, const int* mask, double* partial, double* red,
+                   cudaStream_t s) {
+    const int rpp = kThreads / B;
+    const int g = (int)std::min<int64_t>((std::max(nx, nc) + rpp - 1) / rpp, kRedBlocks);
+    sums_kernel<<<g, kThreads, 0, s>>>(nx, nc, B, aty, z, c, x, y, brow, partial);
+    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+    const int nres = run_map(A, B, x, EpiResidual{brow, mask}, partial + (int64_t)3 * g * B, s);
+    errors_kernel<<<4 * B, kThreads, 0, s>>>(g, nres, B, partial, red);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
@@ -1313,17 +1390,20 @@ void launch_set_rows(int64_t n, int B, const double* row, double* out, const int
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
-void launch_aa_save(int64_t nx, int B, const double* x, const double* z, double* w, const int* mode, cudaStream_t s) {
-    aa_save_kernel<<<grid_for(2 * nx * B), kThreads, 0, s>>>(nx, B, x, z, w, mode);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
+// Two CTAs per SM: the 2 m + 1 sums of a CTA cost two synchronisations each, so a
+// thread takes as many rows as that leaves it (m = 10 at one instance of n = 10:
+// 54 us with one row per thread).
+static int aa_grid(int64_t nx, int B) {
+    const int rpp = kThreads / B;
+    return (int)std::min<int64_t>((2 * nx + rpp - 1) / rpp, 2 * 148);
 }
 
-int64_t aa_partial_size(int64_t nx, int B, int m) { return (int64_t)(2 * m + 1) * spmv_grid(2 * nx, B) * B; }
+int64_t aa_partial_size(int64_t nx, int B, int m) { return (int64_t)(2 * m + 1) * aa_grid(nx, B) * B; }
 
 void launch_aa_update(int64_t nx, int B, int m, const double* x, const double* z, const double* w, double* fprev,
                       double* gprev, double* dF, double* dG, const int* mode, const int* slot, double* partial,
                       double* dots, cudaStream_t s) {
-    const int g = spmv_grid(2 * nx, B);
+    const int g = aa_grid(nx, B);
     if (m <= 4)
         aa_update_kernel<4><<<g, kThreads, 0, s>>>(nx, B, m, x, z, w, fprev, gprev, dF, dG, mode, slot, partial);
     else if (m <= 8)
@@ -1350,11 +1430,6 @@ void launch_aa_mix(int64_t nx, int B, int m, double* x, double* z, const double*
 
 void launch_cg_extrapolate(int64_t n, int B, double* y, double* yprev, const int* mode, cudaStream_t s) {
     cg_extrapolate_kernel<<<grid_for(n * B), kThreads, 0, s>>>(n, B, y, yprev, mode);
-    g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
-}
-
-void launch_c_minus_z(int64_t n, int B, const double* c, double* z, const int* mask, cudaStream_t s) {
-    c_minus_z_kernel<<<grid_for(n * B), kThreads, 0, s>>>(n, B, c, z, mask);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 

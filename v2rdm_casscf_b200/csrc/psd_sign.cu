@@ -9,7 +9,7 @@
 // take every lifted eigenvalue to +-1 to rounding (the last are Newton-Schulz
 // steps).  Y = S X = |S| and Q = Y X give D = S - Q = S (1 - X^2), whose norm
 // bounds the error: an eigenvalue too small to be lifted leaves at most itself.
-// Above the tolerance, eight more lifts and a finish follow, up to kMaxLifts in
+// Above the tolerance, four more lifts and a finish follow, up to kMaxLifts in
 // all (2.46^40 = 4e15).  The projections are (Y + Q) / 2 and (Y - Q) / 2, both
 // positive semidefinite for any X with eigenvalues in [-1, 1] of the right sign.
 // Products are symmetric: upper tiles only, mirrored when they are stored.
@@ -27,7 +27,7 @@ namespace v2g {
 namespace {
 
 constexpr int kFinish = 6;
-constexpr int kFirstLifts = 10, kMoreLifts = 8, kMaxLifts = 40;
+constexpr int kFirstLifts = 10, kMoreLifts = 4, kMaxLifts = 40;
 // a X - b X^3 of the lift (a = 1.5 sqrt(3 c), b = a c for c = 0.9) and of the
 // finish steps (c = 1 / (1 + l + l^2) for the lower end l, from 0.246 on)
 __constant__ double kLift[2] = {2.4647515087732476, 2.2182763578959230};
@@ -77,15 +77,19 @@ __device__ __forceinline__ int next_hint(int hint, int lifts, int rounds) {
 // 0.08 ms per outer iteration, although Jacobi started from its previous
 // eigenvectors there.  Error against 64-bit eigh 1.8e-15 (Jacobi 2.9e-15).
 
-constexpr int kSmallThreads = 512;
-constexpr int kSmallWarps = kSmallThreads / 32;
-constexpr int kSmallTiles = 3;  // 8 x 8 tiles per warp: 36 upper tiles at n = 64
+// WARPS = 16 alone on its SM; 8 beside the team kernel below, whose CTAs come
+// to lie on every SM and leave registers for a CTA of 256 threads only (with 512
+// the small blocks ran after the large ones: 0.47 instead of 0.38 ms for the
+// projection of n = 10).
+constexpr int kSmallWarps = 16, kSmallWarpsBeside = 8;
+// 8 x 8 tiles per warp: 36 upper tiles at n = 64
+__host__ __device__ constexpr int small_tile_count(int warps) { return (36 + warps - 1) / warps; }
 
 // One warp's upper tiles of C = P Q (symmetric, commuting operands with zero
 // padding), as accumulators: tile u covers rows 8 ti[u].., columns 8 tj[u]...
-template <int NU>
-__device__ __forceinline__ void small_tiles(const double* P, const double* Q, int n8, int ld, const int (&ti)[kSmallTiles],
-                                            const int (&tj)[kSmallTiles], double (&acc)[kSmallTiles][2]) {
+template <int NU, int T>
+__device__ __forceinline__ void small_tiles(const double* P, const double* Q, int n8, int ld, const int (&ti)[T],
+                                            const int (&tj)[T], double (&acc)[T][2]) {
     const int lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
     const double *a[NU], *b[NU];
 #pragma unroll
@@ -111,24 +115,29 @@ __device__ __forceinline__ void small_tiles(const double* P, const double* Q, in
     }
 }
 
+template <int T>
 __device__ __forceinline__ void small_product(const double* P, const double* Q, int n8, int ld, int nu,
-                                              const int (&ti)[kSmallTiles], const int (&tj)[kSmallTiles],
-                                              double (&acc)[kSmallTiles][2]) {
-    if (nu == 1)
-        small_tiles<1>(P, Q, n8, ld, ti, tj, acc);
-    else if (nu == 2)
-        small_tiles<2>(P, Q, n8, ld, ti, tj, acc);
-    else if (nu == 3)
-        small_tiles<3>(P, Q, n8, ld, ti, tj, acc);
+                                              const int (&ti)[T], const int (&tj)[T], double (&acc)[T][2]) {
+    switch (nu) {
+        case 1: small_tiles<1>(P, Q, n8, ld, ti, tj, acc); break;
+        case 2: small_tiles<2>(P, Q, n8, ld, ti, tj, acc); break;
+        case 3: small_tiles<3>(P, Q, n8, ld, ti, tj, acc); break;
+        case 4:
+            if constexpr (T >= 4) small_tiles<4>(P, Q, n8, ld, ti, tj, acc);
+            break;
+        case 5:
+            if constexpr (T >= 5) small_tiles<5>(P, Q, n8, ld, ti, tj, acc);
+            break;
+    }
 }
 
 // f(row, col, u, h) for the elements of the warp's tiles that are on or above
 // the diagonal of the matrix
-template <class F>
-__device__ __forceinline__ void small_each(int nu, const int (&ti)[kSmallTiles], const int (&tj)[kSmallTiles], F&& f) {
+template <int T, class F>
+__device__ __forceinline__ void small_each(int nu, const int (&ti)[T], const int (&tj)[T], F&& f) {
     const int lane = threadIdx.x & 31, r = lane >> 2, c = 2 * (lane & 3);
 #pragma unroll
-    for (int u = 0; u < kSmallTiles; u++)
+    for (int u = 0; u < T; u++)
         if (u < nu) {
 #pragma unroll
             for (int h = 0; h < 2; h++) {
@@ -140,12 +149,14 @@ __device__ __forceinline__ void small_each(int nu, const int (&ti)[kSmallTiles],
 
 // hint (optional, one word per task): lifts that sufficed last time in the low
 // byte, calls since the last trial of fewer above it.
-__global__ void __launch_bounds__(kSmallThreads, 1)
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, WARPS == kSmallWarps ? 1 : 2)
     small_sign_kernel(const BlockTask* __restrict__ tasks, int B, const double* __restrict__ aty,
                       const double* __restrict__ c, double* x, double* z, const double* __restrict__ mu,
                       const int* __restrict__ mask, int* __restrict__ hint) {
+    constexpr int kT = small_tile_count(WARPS), kThreads = 32 * WARPS;
     extern __shared__ __align__(16) double sm[];
-    __shared__ double red[kSmallWarps];
+    __shared__ double red[WARPS];
     const BlockTask t = tasks[blockIdx.x];
     const int b = t.inst;
     if (mask && !mask[b]) return;
@@ -153,10 +164,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     double *S = sm, *X = S + n8 * ld, *X2 = X + n8 * ld, *A = X2 + n8 * ld;
     const double m = mu[b];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int ti[kSmallTiles], tj[kSmallTiles], nu = 0;
+    int ti[kT], tj[kT], nu = 0;
 #pragma unroll
-    for (int u = 0; u < kSmallTiles; u++) {
-        int k = warp + u * kSmallWarps, i = 0;
+    for (int u = 0; u < kT; u++) {
+        int k = warp + u * WARPS, i = 0;
         ti[u] = tj[u] = 0;
         if (k < nt * (nt + 1) / 2) {
             while (k >= nt - i) k -= nt - i++;
@@ -166,7 +177,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
         }
     }
     // U = sym(A^T y - c + mu x), zero padded
-    for (int i = threadIdx.x; i < n8 * n8; i += kSmallThreads) {
+    for (int i = threadIdx.x; i < n8 * n8; i += kThreads) {
         const int p = i / n8, q = i % n8;
         double v = 0.0;
         if (p < N && q < N) {
@@ -180,7 +191,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     // the smaller of the Frobenius and the row-sum norm, rounded up to a power
     // of two: scaling by it is exact
     double f = 0.0, rmax = 0.0;
-    for (int p = warp; p < N; p += kSmallWarps) {
+    for (int p = warp; p < N; p += WARPS) {
         double rs = 0.0;
         for (int q = lane; q < N; q += 32) {
             const double v = S[p * ld + q];
@@ -194,7 +205,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     __syncthreads();
     if (lane == 0) red[warp] = rmax;
     __syncthreads();
-    for (int i = 0; i < kSmallWarps; i++)
+    for (int i = 0; i < WARPS; i++)
         if (red[i] > rmax || red[i] != red[i]) rmax = red[i];
     double nrm = rmax;
     if (f > 1e-280 && f < 1e280) nrm = fmin(nrm, sqrt(f));
@@ -206,11 +217,11 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     if (!(nrm > 0.0) || !(nrm <= DBL_MAX)) {
         // a zero block, or one with a non-finite entry
         const double v = nrm == 0.0 ? 0.0 : nan("");
-        for (int i = threadIdx.x; i < N * N; i += kSmallThreads) store(i / N, i % N, v, v);
+        for (int i = threadIdx.x; i < N * N; i += kThreads) store(i / N, i % N, v, v);
         return;
     }
     const int ex = ilogb(nrm) + 1;
-    for (int i = threadIdx.x; i < n8 * n8; i += kSmallThreads) {
+    for (int i = threadIdx.x; i < n8 * n8; i += kThreads) {
         const int o = (i / n8) * ld + i % n8;
         const double v = scalbn(S[o], -ex);
         S[o] = v;
@@ -220,7 +231,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     if (!(f > 0.0 && f <= DBL_MAX)) f = 1.0;
     const double tol = 1e-15 * sqrt((double)N) * f;
     __syncthreads();
-    double acc[kSmallTiles][2];
+    double acc[kT][2];
     // X <- a X - b X^3
     const auto step = [&](double ca, double cb) {
         small_product(X, X, n8, ld, nu, ti, tj, acc);
@@ -541,8 +552,10 @@ void set_sign_attrs() {
     static std::vector<char> done;
     std::lock_guard<std::mutex> lk(mu);
     if ((size_t)dev < done.size() && done[dev]) return;
-    if (cudaFuncSetAttribute(small_sign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) !=
+    if (cudaFuncSetAttribute(small_sign_kernel<kSmallWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) !=
             cudaSuccess ||
+        cudaFuncSetAttribute(small_sign_kernel<kSmallWarpsBeside>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             kSmallSmem) != cudaSuccess ||
         cudaFuncSetAttribute(team_sign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTeamSmem) != cudaSuccess)
         return;
     if ((size_t)dev >= done.size()) done.resize(dev + 1, 0);
@@ -552,12 +565,16 @@ void set_sign_attrs() {
 }  // namespace
 
 void launch_small_project(const BlockTask* tasks, int ntasks, int max_n, int B, const double* aty, const double* c,
-                          double* x, double* z, const double* mu, const int* mask, cudaStream_t s, int* hint) {
+                          double* x, double* z, const double* mu, const int* mask, cudaStream_t s, int* hint, bool beside) {
     if (ntasks == 0) return;
     set_sign_attrs();
     const int n8 = (max_n + 7) / 8 * 8;
     const int smem = 4 * n8 * (n8 + 4) * (int)sizeof(double);
-    small_sign_kernel<<<ntasks, kSmallThreads, smem, s>>>(tasks, B, aty, c, x, z, mu, mask, hint);
+    if (beside)
+        small_sign_kernel<kSmallWarpsBeside>
+            <<<ntasks, 32 * kSmallWarpsBeside, smem, s>>>(tasks, B, aty, c, x, z, mu, mask, hint);
+    else
+        small_sign_kernel<kSmallWarps><<<ntasks, 32 * kSmallWarps, smem, s>>>(tasks, B, aty, c, x, z, mu, mask, hint);
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 

@@ -404,7 +404,7 @@ class GroupRun {
         nact_.alloc(8);  // counters: CG, Jacobi, refinement, fallback, restart
         hnact_buf_.alloc(9);
         hnact_ = hnact_buf_.p;
-        hnact_[8] = 0;
+        hnact_[7] = hnact_[8] = 0;
         stage_.alloc(one_shot_ ? 1 << 16 : 1 << 20);
         mA_ = T.A();
         mAT_ = T.AT();
@@ -412,7 +412,6 @@ class GroupRun {
         upload_state();
         if (one_shot_) return;
         atp_.alloc(X);
-        ax_.alloc(C);
         bv_.alloc(C);
         r_.alloc(C);
         p_.alloc(C);
@@ -524,7 +523,7 @@ class GroupRun {
             CK(cudaEventRecord(ev_fork_, s_));
             CK(cudaStreamWaitEvent(s_small_, ev_fork_, 0));
             launch_small_project(small_d_.p, nsmall_, max_small_, B_, aty_.p, c_.p, x_.p, z_.p, mu_.p, mask_.p,
-                                 s_small_, small_hint_.p);
+                                 s_small_, small_hint_.p, sign_grid_ > 0);
             CK(cudaEventRecord(ev_join_, s_small_));
         }
         project_large(rho);
@@ -656,8 +655,9 @@ class GroupRun {
         launch_lam_from_diag(large_d_.p, nlarge_, W_.p, bjac_.p, lam_.p, s_);
     }
 
-    // After a synchronisation of the stream.
-    void check_projection() const {
+    // After a synchronisation of the stream: did the cooperative kernels finish.
+    void check_waits() const {
+        if (hnact_[7] != 0) throw CudaError("an exchange of the persistent CG did not complete (wait ran out)");
         if (hnact_[8] != 0) throw CudaError("a team of the projection did not meet (wait ran out)");
     }
 
@@ -760,14 +760,12 @@ class GroupRun {
                 // w = the (x, z) this step starts from
                 for (int b = 0; b < B_; b++) aa.mode[b] = (active[b] && aa_memory(b) > 0) ? 1 : 0;
                 put(amode_.p, aa.mode.data(), B_);
-                launch_aa_save(nx_, B_, x_.p, z_.p, aw_.p, amode_.p, s_);
             }
             std::fill(mu_changed.begin(), mu_changed.end(), 0);
             CK(cudaEventRecord(e0, s_));
-            // Ax = -tau mu (A x - b); z <- c - z; B = A z + Ax   (:1783-1794)
-            launch_spmv(mA_, B_, x_.p, ax_.p, T_.b.p, coef_.p, nullptr, mask_.p, s_);
-            launch_c_minus_z(nx_, B_, c_.p, z_.p, mask_.p, s_);
-            launch_spmv(mA_, B_, z_.p, bv_.p, nullptr, nullptr, ax_.p, mask_.p, s_);
+            // B = A (c - z) - tau mu (A x - b) (:1783-1794), the state w kept
+            launch_rhs(mA_, nx_, B_, c_.p, x_.p, z_.p, T_.b.p, coef_.p, mask_.p, aa_m_ > 0 ? aw_.p : nullptr,
+                       amode_.p, bv_.p, s_);
             // CG tolerance (:1797-1805)
             for (int b = 0; b < B_; b++) {
                 const Options& o = opt(b);
@@ -814,17 +812,14 @@ class GroupRun {
             project(rho, mixed);
             CK(cudaEventRecord(e2, s_));
             // ed = ||A^T y + z - c||, ep = ||A x - b||, E = c.x, b.y (:1826-1852)
-            launch_reduce(RED_ED, nx_, B_, aty_.p, z_.p, c_.p, nullptr, partial_.p, red_.p, s_);
-            launch_spmv(mA_, B_, x_.p, ax_.p, nullptr, nullptr, nullptr, mask_.p, s_);
-            launch_reduce(RED_EP, nc_, B_, ax_.p, nullptr, nullptr, T_.b.p, partial_.p, red_.p + B_, s_);
-            launch_reduce(RED_DOT, nx_, B_, c_.p, x_.p, nullptr, nullptr, partial_.p, red_.p + 2 * B_, s_);
-            launch_reduce(RED_DOT_ROW, nc_, B_, y_.p, nullptr, nullptr, T_.b.p, partial_.p, red_.p + 3 * B_, s_);
+            launch_errors(mA_, nx_, nc_, B_, aty_.p, x_.p, y_.p, z_.p, c_.p, T_.b.p, mask_.p, partial_.p, red_.p,
+                          s_);
             CK(cudaMemcpyAsync(hscal_, red_.p, 4 * B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
             if (tc_) tc_gemm_status_async(hnact_ + 5, s_);
             CK(cudaStreamSynchronize(s_));
             stage_synced();
             std::copy(hcs_, hcs_ + B_, cs.begin());
-            check_projection();
+            check_waits();
             if (tc_ && hnact_[5] != 0)
                 throw CudaError("a tensor-core GEMM of the projection did not finish (pipeline wait ran out)");
             float ms_cg = 0, ms_xz = 0;
@@ -1000,7 +995,7 @@ class GroupRun {
         const DevBuf<double>* vecs[3] = {&y_, &x_, &z_};
         const int64_t lens[3] = {nc_, nx_, nx_};
         for (int k = 0; k < 3; k++) {
-            launch_reduce(RED_DOT, lens[k], B_, vecs[k]->p, vecs[k]->p, nullptr, nullptr, partial_.p, red_.p, s_);
+            launch_dot(lens[k], B_, vecs[k]->p, vecs[k]->p, partial_.p, red_.p, s_);
             CK(cudaMemcpyAsync(&sums[k * B_], red_.p, B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
         }
         double gmax = 0.0;
@@ -1031,7 +1026,7 @@ class GroupRun {
         const DevBuf<double>* vecs[3] = {&y_, &x_, &z_};
         const int64_t lens[3] = {nc_, nx_, nx_};
         for (int k = 0; k < 3; k++) {
-            launch_reduce(RED_DOT, lens[k], B_, vecs[k]->p, vecs[k]->p, nullptr, nullptr, partial_.p, red_.p, s_);
+            launch_dot(lens[k], B_, vecs[k]->p, vecs[k]->p, partial_.p, red_.p, s_);
             CK(cudaMemcpyAsync(&sums[k], red_.p + b, sizeof(double), cudaMemcpyDeviceToHost, s_));
             CK(cudaStreamSynchronize(s_));
         }
@@ -1085,6 +1080,7 @@ class GroupRun {
         std::vector<double> dmu(B_);
         CK(cudaMemcpyAsync(dmu.data(), mu_.p, B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
         CK(cudaStreamSynchronize(s_));
+        check_waits();
         for (int b = 0; b < B_; b++)
             if (fs[b]) dmu[b] = fs[b] == 2 ? mu[b] : 1.0;
         CK(cudaMemcpyAsync(mu_.p, dmu.data(), B_ * sizeof(double), cudaMemcpyHostToDevice, s_));
@@ -1127,7 +1123,7 @@ class GroupRun {
                 CK(cudaEventCreate(&e1));
             }
             const double* in = which == 0 ? x_.p : y_.p;
-            double* out = which == 0 ? ax_.p : aty_.p;
+            double* out = which == 0 ? bv_.p : aty_.p;
             float best = 0.f;
             int bestv = -1;
             for (int v = 0; v < kMapVariants; v++) {
@@ -1225,19 +1221,15 @@ class GroupRun {
     void cg_solve() {
         // Small groups (outside profile mode): the whole solve in one
         // cooperative launch, the phases of each iteration separated by grid
-        // exchanges (maps.cu), one host synchronisation per solve
+        // exchanges (maps.cu)
         if (!profile_ && loop_grid_ > 0) {
             int cap = 1;
             for (auto* p : P_) cap = std::max(cap, p->opt.cg_maxiter);
             cap += 2;
             CK(launch_cg_loop(mA_, mAT_, B_, bv_.p, y_.p, r_.p, p_.p, atp_.p, cs_.p, loopslots_.p, looperr_.p,
                               nact_.p, nact_.p + 6, cap, loop_grid_, s_));
-            CK(cudaMemcpyAsync(hnact_, nact_.p, sizeof(int), cudaMemcpyDeviceToHost, s_));
-            CK(cudaMemcpyAsync(hnact_ + 6, nact_.p + 6, sizeof(int), cudaMemcpyDeviceToHost, s_));
+            // no synchronisation: the flag is read with the iteration's results
             CK(cudaMemcpyAsync(hnact_ + 7, looperr_.p, sizeof(int), cudaMemcpyDeviceToHost, s_));
-            CK(cudaStreamSynchronize(s_));
-            if (hnact_[7] != 0) throw CudaError("an exchange of the persistent CG did not complete (wait ran out)");
-            cg_loop_iters_ += hnact_[6];
             return;  // cap iterations stop every instance by its own CG_MAXITER
         }
         // q = A^T y, r = rhs - A q
@@ -1586,7 +1578,7 @@ class GroupRun {
     cudaStream_t s_ = nullptr;
     cudaStream_t s_small_ = nullptr;  // the small blocks' projection, beside the large blocks'
     cudaEvent_t ev_fork_ = nullptr, ev_join_ = nullptr;
-    DevBuf<double> c_, x_, z_, aty_, atp_, y_, ax_, bv_, r_, p_, partial_, red_, mu_, coef_;
+    DevBuf<double> c_, x_, z_, aty_, atp_, y_, bv_, r_, p_, partial_, red_, mu_, coef_;
     DevBuf<int> mask_, nact_, smask1_, smask2_;
     DevBuf<CgScalars> cs_;
     // CG start extrapolation (cg_extrapolate): the previous CG start and the
@@ -1650,7 +1642,6 @@ class GroupRun {
     int loop_grid_ = 0;
     DevBuf<unsigned long long> loopslots_;
     DevBuf<int> looperr_;
-    long cg_loop_iters_ = 0;
     cudaGraphExec_t cg_loop_exec_ = nullptr;  // the device-side CG loop (WHILE node)
     long cg_loop_nodes_ = 0;
     bool cg_loop_ok_ = true;
@@ -2104,7 +2095,7 @@ int v2g_update_xz(v2g_handle* h, double mu) {
         g.project();
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(g.stream()));
-        g.check_projection();
+        g.check_waits();
         g.download_state();
         return V2G_OK;
     });
