@@ -16,6 +16,7 @@
 #include <cooperative_groups.h>
 
 #include <cfloat>
+#include <cstdint>
 
 #include <mutex>
 #include <vector>
@@ -210,15 +211,10 @@ __global__ void cold_start_kernel(const BlockTask* __restrict__ tasks, const dou
     }
 }
 
-// C = op(A) diag(d) op(B) on 64 x 64 tiles of the padded workspaces.
-// S x S threads per tile (S = 64 / R), each holding an R x R block of C in
-// registers (rows ty + S i, columns tx + S j).  R = 8 (64 threads): 16
-// shared-memory loads feed 64 FMAs, which matches the FP64 FMA rate to the
-// shared-memory bandwidth; the launch for large grids.  R = 4 (256 threads):
-// four times the warps per tile and a quarter of the serial FMA chain per
-// thread, for grids too small to fill the GPU (one instance's few blocks),
-// where the kernel is latency-bound.  The K loop is double buffered through
-// registers; every C entry is one FMA chain in k order in both forms.
+// C = op(A) diag(d) op(B) on 64 x 64 tiles of the padded workspaces, with
+// 8-byte loads (buffers of any alignment): 16 x 16 threads per tile, each
+// holding a 4 x 4 block of C in registers (rows ty + 16 i, columns tx + 16 j).
+// The K loop is double buffered through registers.
 constexpr int kGemmBK = 16;
 constexpr int kGemmLd = 64 + 1;
 
@@ -274,15 +270,14 @@ __device__ __forceinline__ void gemm_store_chunk(double (*As)[kGemmLd], double (
     }
 }
 
-template <int R>
-__global__ void __launch_bounds__((64 / R) * (64 / R)) gemm_kernel(const BlockTask* __restrict__ tasks,
+__global__ void __launch_bounds__(256) gemm_kernel(const BlockTask* __restrict__ tasks,
                                                                    const GemmTile* __restrict__ tiles,
                                                                    const double* __restrict__ A, int transA,
                                                                    const double* __restrict__ Bm, int transB,
                                                                    const double* __restrict__ dvec,
                                                                    double* __restrict__ C,
                                                                    const int* __restrict__ bmask) {
-    constexpr int S = 64 / R, NT = S * S, U = 1024 / NT;
+    constexpr int R = 4, S = 64 / R, NT = S * S, U = 1024 / NT;
     __shared__ double As[2][kGemmBK][kGemmLd];
     __shared__ double Bs[2][kGemmBK][kGemmLd];
     const GemmTile tl = tiles[blockIdx.x];
@@ -332,12 +327,123 @@ __global__ void __launch_bounds__((64 / R) * (64 / R)) gemm_kernel(const BlockTa
         for (int j = 0; j < R; j++) cc[(int64_t)(i0 + ty + S * i) * np + j0 + tx + S * j] = acc[i][j];
 }
 
+// The same product on the FP64 tensor instructions (mma.sync m8n8k4; tcgen05
+// has no FP64 kind), for 16-byte aligned workspaces: 64 x 64 tiles, eight warps
+// of 32 x 16 each, operands as they lie in memory ([row][k] or [k][row]) in a
+// three-stage cp.async ring whose leading dimensions (20 and 68 doubles) put
+// the 16 lanes of a half-warp on 16 banks.  Bound: the FP64 rate, 64 FMAs per
+// cycle and SM, against which gemm_kernel spends a shared load per two FMAs.
+constexpr int kDmBK = 16, kDmRing = 3;
+constexpr int kDmRowLd = kDmBK + 4, kDmColLd = 64 + 4;
+constexpr int kDmOperand = 64 * kDmRowLd > kDmBK * kDmColLd ? 64 * kDmRowLd : kDmBK * kDmColLd;
+constexpr int kDmStage = 2 * kDmOperand + kDmBK;  // A, B and the chunk of d
+constexpr size_t kDmSmem = kDmRing * kDmStage * sizeof(double);
+
+__device__ __forceinline__ void dm_copy16(double* dst, const double* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// 64 x kDmBK elements (row i0 + i, k0 + k) of an operand: stored [k][row] when BYK
+template <bool BYK>
+__device__ __forceinline__ void dm_fetch(double* dst, const double* src, int np, int i0, int k0) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int e = threadIdx.x + 256 * h;
+        if (BYK) {
+            const int k = e >> 5, i = 2 * (e & 31);
+            dm_copy16(dst + k * kDmColLd + i, src + (int64_t)(k0 + k) * np + i0 + i);
+        } else {
+            const int i = e >> 3, k = 2 * (e & 7);
+            dm_copy16(dst + i * kDmRowLd + k, src + (int64_t)(i0 + i) * np + k0 + k);
+        }
+    }
+}
+
+// TA: op(A) = A^T, so A lies [k][row]; TB: op(B) = B^T, so B lies [column][k]
+template <bool TA, bool TB>
+__global__ void __launch_bounds__(256, 2) gemm_dmma_kernel(const BlockTask* __restrict__ tasks,
+                                                           const GemmTile* __restrict__ tiles,
+                                                           const double* __restrict__ A, const double* __restrict__ Bm,
+                                                           const double* __restrict__ dvec, double* __restrict__ C,
+                                                           const int* __restrict__ bmask) {
+    extern __shared__ __align__(16) double dm[];
+    const GemmTile tl = tiles[blockIdx.x];
+    if (bmask && !bmask[tl.task]) return;
+    const BlockTask t = tasks[tl.task];
+    const int np = t.np, i0 = tl.ti * 64, j0 = tl.tj * 64;
+    const double* a = A + t.woff;
+    const double* b = Bm + t.woff;
+    const double* d = dvec ? dvec + t.doff : nullptr;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
+    const int wr = 32 * (warp & 1), wc = 16 * (warp >> 1);
+    const int nk = np / kDmBK;
+    auto fetch = [&](int kc) {
+        if (kc < nk) {
+            double* s = dm + (kc % kDmRing) * kDmStage;
+            dm_fetch<TA>(s, a, np, i0, kc * kDmBK);
+            dm_fetch<!TB>(s + kDmOperand, b, np, j0, kc * kDmBK);
+            if (d && threadIdx.x < kDmBK / 2)
+                dm_copy16(s + 2 * kDmOperand + 2 * threadIdx.x, d + kc * kDmBK + 2 * threadIdx.x);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[4][2][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+    fetch(0);
+    fetch(1);
+    for (int kc = 0; kc < nk; kc++) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        fetch(kc + 2);
+        const double* As = dm + (kc % kDmRing) * kDmStage;
+        const double* Bs = As + kDmOperand;
+        const double* ds = Bs + kDmOperand;
+#pragma unroll
+        for (int kk = 0; kk < kDmBK; kk += 4) {
+            double av[4], bv[2];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int row = wr + 8 * i + r;
+                av[i] = TA ? As[(kk + c) * kDmColLd + row] : As[row * kDmRowLd + kk + c];
+            }
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int col = wc + 8 * j + r;
+                bv[j] = TB ? Bs[col * kDmRowLd + kk + c] : Bs[(kk + c) * kDmColLd + col];
+            }
+            if (d) {
+                const double dk = ds[kk + c];
+#pragma unroll
+                for (int i = 0; i < 4; i++) av[i] *= dk;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                        : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+                        : "d"(av[i]), "d"(bv[j]));
+        }
+    }
+    double* cc = C + t.woff;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            *reinterpret_cast<double2*>(cc + (int64_t)(i0 + wr + 8 * i + r) * np + j0 + wc + 8 * j + 2 * c) =
+                make_double2(acc[i][j][0], acc[i][j][1]);
+}
+
 // Split-K form for the smallest grids (one instance's few blocks): a cluster
 // of kSplitK CTAs per 64 x 64 tile, CTA r of the cluster summing k in
-// [r np / kSplitK, (r + 1) np / kSplitK) as gemm_kernel<4> does; the partial
+// [r np / kSplitK, (r + 1) np / kSplitK) as gemm_kernel does; the partial
 // tiles meet in rank 0's registers through distributed shared memory, added
 // in rank order (a fixed order: no atomics, no second launch).  kSplitK times
-// the CTAs of gemm_kernel<4>, each with a quarter of the FMA chain.
+// the CTAs of gemm_kernel, each with a quarter of the FMA chain.
 constexpr int kSplitK = 4;
 __global__ void __cluster_dims__(kSplitK, 1, 1) __launch_bounds__(256)
     gemm_splitk_kernel(const BlockTask* __restrict__ tasks, const GemmTile* __restrict__ tiles,
@@ -1006,6 +1112,9 @@ void set_smem_attrs() {
                                     (int)kJacobiSmem) == cudaSuccess;
     ok = ok && cudaFuncSetAttribute(bj_update_wv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)kJacobiSmem) == cudaSuccess;
+    for (auto k : {gemm_dmma_kernel<false, false>, gemm_dmma_kernel<false, true>, gemm_dmma_kernel<true, false>,
+                   gemm_dmma_kernel<true, true>})
+        ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDmSmem) == cudaSuccess;
     if (!ok) return;
     if ((size_t)dev >= done.size()) done.resize(dev + 1, 0);
     done[dev] = 1;
@@ -1030,15 +1139,22 @@ void launch_cold_start(const BlockTask* tasks, int ntasks, int max_np, const dou
 void launch_gemm(const BlockTask* tasks, const GemmTile* tiles, int ntiles, const double* A, bool transA,
                  const double* Bm, bool transB, const double* dvec, double* C, const int* bmask, cudaStream_t s) {
     if (ntiles == 0) return;
-    // below two tiles per SM (148 SMs) the 256-thread form hides the latency
-    // the 64-thread form cannot; below half a tile per SM, the split-K
-    // clusters also spread each tile's K over four CTAs
-    if (ntiles * kSplitK <= 2 * 148)
+    set_smem_attrs();
+    // up to half a tile per SM the split-K clusters spread each tile's K over
+    // four CTAs (the blocks of one n = 10 instance 14.6 us, tensor form 16.5);
+    // above, the tensor form (five n = 13 instances 94 -> 62 us, 19 blocks of 800
+    // 1,026 -> 802, 21.3 -> 27.3 TFLOP/s, one of 5,000 27.8), unless a caller's
+    // buffer is not 16-byte aligned
+    const bool aligned = (((uintptr_t)A | (uintptr_t)Bm | (uintptr_t)C | (uintptr_t)dvec) & 15) == 0;
+    if (ntiles * kSplitK <= 2 * 148) {
         gemm_splitk_kernel<<<ntiles * kSplitK, 256, 0, s>>>(tasks, tiles, A, transA, Bm, transB, dvec, C, bmask);
-    else if (ntiles < 2 * 148)
-        gemm_kernel<4><<<ntiles, 256, 0, s>>>(tasks, tiles, A, transA, Bm, transB, dvec, C, bmask);
-    else
-        gemm_kernel<8><<<ntiles, 64, 0, s>>>(tasks, tiles, A, transA, Bm, transB, dvec, C, bmask);
+    } else if (aligned) {
+        auto k = transA ? (transB ? gemm_dmma_kernel<true, true> : gemm_dmma_kernel<true, false>)
+                        : (transB ? gemm_dmma_kernel<false, true> : gemm_dmma_kernel<false, false>);
+        k<<<ntiles, 256, kDmSmem, s>>>(tasks, tiles, A, Bm, dvec, C, bmask);
+    } else {
+        gemm_kernel<<<ntiles, 256, 0, s>>>(tasks, tiles, A, transA, Bm, transB, dvec, C, bmask);
+    }
     g_kernel_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
