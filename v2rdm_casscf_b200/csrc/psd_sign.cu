@@ -52,17 +52,29 @@ __device__ double cta_total(double v, double* red) {
     return s;
 }
 
-// The hint for the next call: the lifts that sufficed, where a finish lifts as
-// much as four lifts; every eighth call tries two fewer.
-__device__ __forceinline__ int next_hint(int hint, int lifts, int rounds) {
-    int k = lifts + 4 * (rounds - 1), calls = (hint >> 8) + 1;
-    if (k > kMaxLifts) k = kMaxLifts;
-    if (rounds > 1) calls = 0;
-    if (calls == 8) {
-        k = k > 4 ? k - 2 : 2;
-        calls = 0;
+// The hint for the next call, from this call's (0: none yet) and its rounds: the
+// lifts to begin with in the low byte, calls (plus 16) until the next trial in
+// the second, and whether this count is a trial.  Every eighth call tries one
+// lift fewer; a failed trial goes back and waits 24 calls, and where a count
+// that was no trial fails (the tolerance or the spectrum moved), four more, the
+// next round's lifts.
+__device__ __forceinline__ int next_hint(int hint, int rounds) {
+    int k = (hint & 255) ? (hint & 255) : kFirstLifts, calls = hint ? ((hint >> 8) & 255) - 16 : 0;
+    int trial = hint >> 16;
+    if (rounds == 1) {
+        trial = 0;
+        if (++calls >= 8) {
+            trial = k > 2;
+            k -= trial;
+            calls = 0;
+        }
+    } else {
+        k = trial ? k + 1 : k + 4 * (rounds - 1);
+        calls = trial ? -16 : 0;
+        trial = 0;
+        if (k > kMaxLifts) k = kMaxLifts;
     }
-    return k | calls << 8;
+    return k | (calls + 16) << 8 | trial << 16;
 }
 
 // ---- blocks of dimension up to 64: one CTA, everything in shared memory ----
@@ -147,8 +159,7 @@ __device__ __forceinline__ void small_each(int nu, const int (&ti)[T], const int
         }
 }
 
-// hint (optional, one word per task): lifts that sufficed last time in the low
-// byte, calls since the last trial of fewer above it.
+// hint (optional, one word per task): see next_hint.
 template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS, WARPS == kSmallWarps ? 1 : 2)
     small_sign_kernel(const BlockTask* __restrict__ tasks, int B, const double* __restrict__ aty,
@@ -267,7 +278,7 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS == kSmallWarps ? 1 : 2)
         if (d2 <= tol * tol || lifts >= kMaxLifts) break;
         more = kMoreLifts;
     }
-    if (hint && threadIdx.x == 0) hint[blockIdx.x] = next_hint(h0, lifts, rounds);
+    if (hint && threadIdx.x == 0) hint[blockIdx.x] = next_hint(h0, rounds);
     const double sx = scalbn(0.5, ex) / m, sz = scalbn(0.5, ex);
     small_each(nu, ti, tj, [&](int p, int q, int u, int h) {
         if (q < N) {
@@ -286,12 +297,12 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS == kSmallWarps ? 1 : 2)
 // instance of ten orbitals the latency of a product (first loads 2,000 cycles,
 // a tile's FP64 instructions 1,700 to 3,600, the barrier 3,000); with many
 // or large blocks the FP64 rate.  The operands are symmetric, so both panels of
-// a tile are rows: 32 x 32 chunks through a three-stage cp.async ring (L2 only:
+// a tile are rows: 32 x 32 chunks through a four-stage cp.async ring (L2 only:
 // other CTAs wrote them).  One projection of ten orbitals (blocks of 100 to 200,
 // 34 to 60 products) takes 0.3 ms on a B200, of fifteen (225 to 450) 0.9 ms;
 // block Jacobi took 8.0 and 22 ms from cold, at twice the error.
 constexpr int kTeamThreads = 256;
-constexpr int kTile = 32, kChunkLd = kTile + 4, kRing = 3;
+constexpr int kTile = 32, kChunkLd = kTile + 4, kRing = 4;
 constexpr int kChunk = kTile * kChunkLd;  // one operand's chunk in shared memory
 constexpr long kTeamPolls = 1L << 25;     // about a second of polling (short sleeps)
 
@@ -329,11 +340,14 @@ __device__ __forceinline__ void cp_wait() {
 }
 
 // The CTA's share of the upper 32 x 32 tiles of C = P Q (n32 x n32, leading
-// dimension ld, symmetric commuting operands): f(row, col, value) for every
-// element on or above the diagonal.
-template <class F>
+// dimension ld, symmetric commuting operands): f(row, col, value, e) for every
+// element on or above the diagonal, with e = E(row, col) loaded before the K
+// loop.  Even and odd K steps of four go to accumulators of their own: two
+// chains per element keep eight instructions in flight per SM quarter, with one
+// the loop ran at half the FP64 rate.
+template <class E, class F>
 __device__ __forceinline__ void team_product(const double* P, const double* Q, int ld, int n32, int rank, int size,
-                                             double* ring, F&& f) {
+                                             double* ring, E&& early, F&& f) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, c = lane & 3;
     const int wr = 8 * (warp & 3), wc = 16 * (warp >> 2);  // the warp's 8 x 16 part of a tile
     const int nt = n32 / kTile, nk = nt;
@@ -344,45 +358,48 @@ __device__ __forceinline__ void team_product(const double* P, const double* Q, i
         const double* pr = P + (int64_t)ti * kTile * ld;
         const double* qr = Q + (int64_t)tj * kTile * ld;
         auto fetch = [&](int kc) {
-            double* s = ring + (kc % kRing) * 2 * kChunk;
+            if (kc < nk) {
+                double* s = ring + (kc % kRing) * 2 * kChunk;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int e = threadIdx.x + h * kTeamThreads, row = e >> 4, col = 2 * (e & 15);
-                cp_async16(s + row * kChunkLd + col, pr + (int64_t)row * ld + kc * kTile + col);
-                cp_async16(s + kChunk + row * kChunkLd + col, qr + (int64_t)row * ld + kc * kTile + col);
+                for (int h = 0; h < 2; h++) {
+                    const int e = threadIdx.x + h * kTeamThreads, row = e >> 4, col = 2 * (e & 15);
+                    cp_async16(s + row * kChunkLd + col, pr + (int64_t)row * ld + kc * kTile + col);
+                    cp_async16(s + kChunk + row * kChunkLd + col, qr + (int64_t)row * ld + kc * kTile + col);
+                }
             }
             cp_commit();
         };
-        double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        const int row = ti * kTile + wr + r, col = tj * kTile + wc + 2 * c;
         __syncthreads();  // the ring is free
         fetch(0);
-        if (nk > 1)
-            fetch(1);
-        else
-            cp_commit();
+        fetch(1);
+        fetch(2);
+        double ev[2][2];
+#pragma unroll
+        for (int v = 0; v < 2; v++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) ev[v][h] = early(row, col + 8 * v + h);
+        double acc[2][2][2] = {};
         for (int kc = 0; kc < nk; kc++) {
-            cp_wait<1>();
+            cp_wait<2>();
             __syncthreads();
-            if (kc + 2 < nk)
-                fetch(kc + 2);
-            else
-                cp_commit();
+            fetch(kc + 3);
             const double* a = ring + (kc % kRing) * 2 * kChunk + (wr + r) * kChunkLd + c;
             const double* b = ring + (kc % kRing) * 2 * kChunk + kChunk + (wc + r) * kChunkLd + c;
 #pragma unroll
-            for (int kk = 0; kk < kTile; kk += 4) {
-                const double av = a[kk], b0 = b[kk], b1 = b[8 * kChunkLd + kk];
-                dmma(acc[0][0], acc[0][1], av, b0);
-                dmma(acc[1][0], acc[1][1], av, b1);
-            }
+            for (int kk = 0; kk < kTile; kk += 8)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const double av = a[kk + 4 * h], b0 = b[kk + 4 * h], b1 = b[8 * kChunkLd + kk + 4 * h];
+                    dmma(acc[h][0][0], acc[h][0][1], av, b0);
+                    dmma(acc[h][1][0], acc[h][1][1], av, b1);
+                }
         }
 #pragma unroll
         for (int v = 0; v < 2; v++)
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int row = ti * kTile + wr + r, col = tj * kTile + wc + 8 * v + 2 * c + h;
-                if (row <= col) f(row, col, acc[v][h]);
-            }
+            for (int h = 0; h < 2; h++)
+                if (row <= col + 8 * v + h) f(row, col + 8 * v + h, acc[0][v][h] + acc[1][v][h], ev[v][h]);
     }
 }
 
@@ -487,13 +504,15 @@ __global__ void __launch_bounds__(kTeamThreads, 2) team_sign_kernel(const __grid
             M[(int64_t)p * ld + q] = v;
             M[(int64_t)q * ld + p] = v;
         };
+        const auto none = [](int, int) { return 0.0; };
         // X <- a X - b X^3
         auto step = [&](double ca, double cb) {
-            team_product(X, X, ld, n32, tm.rank, tm.size, ring, [&](int p, int q, double v) { put(A, p, q, v); });
+            team_product(X, X, ld, n32, tm.rank, tm.size, ring, none,
+                         [&](int p, int q, double v, double) { put(A, p, q, v); });
             if (!sync()) return false;
-            team_product(X, A, ld, n32, tm.rank, tm.size, ring, [&](int p, int q, double v) {
-                put(X2, p, q, ca * __ldcg(X + (int64_t)p * ld + q) - cb * v);
-            });
+            team_product(
+                X, A, ld, n32, tm.rank, tm.size, ring, [&](int p, int q) { return __ldcg(X + (int64_t)p * ld + q); },
+                [&](int p, int q, double v, double xv) { put(X2, p, q, ca * xv - cb * v); });
             if (!sync()) return false;
             double* s = X;
             X = X2;
@@ -510,19 +529,22 @@ __global__ void __launch_bounds__(kTeamThreads, 2) team_sign_kernel(const __grid
             lifts += more;
             rounds++;
             // Y = S X (into X2), Q = Y X (into A)
-            team_product(S, X, ld, n32, tm.rank, tm.size, ring, [&](int p, int q, double v) { put(X2, p, q, v); });
+            team_product(S, X, ld, n32, tm.rank, tm.size, ring, none,
+                         [&](int p, int q, double v, double) { put(X2, p, q, v); });
             if (!sync()) return;
             double d2 = 0.0;
-            team_product(X2, X, ld, n32, tm.rank, tm.size, ring, [&](int p, int q, double v) {
-                const double d = __ldcg(S + (int64_t)p * ld + q) - v;
-                d2 += p == q ? d * d : 2.0 * d * d;
-                A[(int64_t)p * ld + q] = v;
-            });
+            team_product(
+                X2, X, ld, n32, tm.rank, tm.size, ring, [&](int p, int q) { return __ldcg(S + (int64_t)p * ld + q); },
+                [&](int p, int q, double v, double sv) {
+                    const double d = sv - v;
+                    d2 += p == q ? d * d : 2.0 * d * d;
+                    A[(int64_t)p * ld + q] = v;
+                });
             if (!team_sum(cta_total(d2, red), d2)) return;
             if (d2 <= tol * tol || lifts >= kMaxLifts) break;
             more = kMoreLifts;
         }
-        if (tm.rank == 0 && threadIdx.x == 0) g.hint[tm.task] = next_hint(h0, lifts, rounds);
+        if (tm.rank == 0 && threadIdx.x == 0) g.hint[tm.task] = next_hint(h0, rounds);
         // every thread takes the tile elements it computed
         const double sx = scalbn(0.5, ex) / m, sz = scalbn(0.5, ex);
         const int nt = n32 / kTile;
