@@ -409,7 +409,7 @@ def run_gpu(args):
         ta, tt = b20.time_maps(19, 20)
         nbytes = 8.0 * (b20.dimx + b20.nconstraints) * 19
         ach = 2 * nbytes / (ta + tt) / 1e9
-        out["roofline_batch"] = {"kernel": "ell_kernel + long_kernel, A and A^T of n = 20 with 19 instances "
+        out["roofline_batch"] = {"kernel": "ell_kernel, A and A^T of n = 20 with 19 instances "
                                            "interleaved (the batched workload's largest group), graph replay",
                                  "bound": "hbm", "achieved": ach, "peak": pk, "peak_kind": pk_kind, "unit": "GB/s",
                                  "frac": ach / pk, "traffic": ROOFLINE_TRAFFIC.get((20, 19)),
@@ -425,15 +425,15 @@ def run_gpu(args):
 
 
 # DRAM bytes (read + write) per launch of the roofline kernels, from one ncu
-# capture of the same launches (profiles/ell_kernel_*.md gives the command):
+# capture of the same launches (profiles/ell_kernel_lanes_traffic.md gives the command):
 # key = (n, instances)
 ROOFLINE_TRAFFIC = {
-    # A 556.5 MB, A^T 763.3 MB (means of 23 launches each), ell_kernel<4, 1>
-    (20, 19): 659.9e6,
-    # H10: A 4.22 MB, A^T 4.15 MB read, nothing written back (ell_kernel<2, 0>);
+    # A 521.3 MB, A^T 715.0 MB
+    (20, 19): 618.1e6,
+    # H10: A 2.15 MB, A^T 2.31 MB read, nothing written back;
     # ncu flushes the caches before each launch, so this is the tables and the
     # input read cold: inside the solve both stay in L2
-    (10, 1): 4.18e6,
+    (10, 1): 2.23e6,
 }
 
 
@@ -483,7 +483,7 @@ def roofline_workload(solvers, pk, pk_kind):
     nbytes = 8.0 * (s.dimx + s.nconstraints)
     ach = 2 * nbytes / (ta + tt) / 1e9
     key = (int(s.active[0]), 1)
-    return {"kernel": "ell_kernel + long_kernel (A and A^T of the CG), one instance of the workload, graph replay",
+    return {"kernel": "ell_kernel (A and A^T of the CG), one instance of the workload, graph replay",
             "bound": "hbm", "achieved": ach, "peak": pk, "peak_kind": pk_kind, "unit": "GB/s", "frac": ach / pk,
             "traffic": ROOFLINE_TRAFFIC.get(key), "bytes_per_launch": nbytes,
             "us_per_launch": {"A": ta * 1e6, "AT": tt * 1e6},
