@@ -13,6 +13,8 @@
 #include <cstdint>
 #include <vector>
 
+#include "map_units.h"
+
 namespace v2g {
 
 // Number of kernels the launchers below have issued (all threads, all devices).
@@ -25,12 +27,7 @@ extern std::atomic<long> g_kernel_launches;
 // (traces, contractions) are kept as CSR, the first nmid of them (at most
 // kMidRow entries, kMidMany or more rows of the same length) reduced by a warp
 // each, the others by a whole CTA.
-constexpr int kMaxBuckets = 7;
-constexpr int kMidRow = 256, kMidMany = 32;
 constexpr int kLongClasses = 5;  // rows of up to 16, 32, 64, 128 and 256 entries
-// maps with fewer rows are bound by latency at small batches: their rows of 17
-// to 32 entries take a warp each too, instead of one thread
-constexpr int kLatencyRows = 1 << 18;
 constexpr int kCodeShift = 27;                 // packed entry: 27 column bits, 4 code bits
 constexpr int kBookSize = 1 << (31 - kCodeShift);  // 16 coefficients at most
 struct DevMap {

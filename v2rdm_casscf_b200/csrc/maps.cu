@@ -113,7 +113,6 @@ constexpr int kWarps = 32;         // of the largest CTA
 // lane: l and l + (B + 1) / 2 for odd B (contiguous 8-byte loads), 2 l and
 // 2 l + 1 for even B (16-byte loads).
 enum LaneMode { kOne = 0, kOdd = 1, kEven = 2 };
-__host__ __device__ constexpr int lanes_of(int B) { return (B + 1) / 2; }
 static LaneMode lane_mode(int B) { return B == 1 ? kOne : ((B & 1) ? kOdd : kEven); }
 
 // Sum of v over the CTA, to thread 0: one synchronisation.  The scratch is free
@@ -131,23 +130,10 @@ __device__ __forceinline__ double cta_sum(double v) {
     return threadIdx.x == 0 ? s : 0.0;
 }
 
-// Work units of one map application: first the long rows (a CTA each), then
-// the mid rows (a warp each, 32 instances at a time), then the row tiles.
-// Unit u runs on CTA u % gridDim.x.
-struct Blocks {
-    int start[kMaxBuckets + 1];  // first unit of each bucket's row tiles; the last: the unit count
-    int mid;                     // first mid-row unit
-    int midchunks;               // instance chunks of 32 per group of mid rows
-    int deep;                    // the deep form: ell_depth(width) rows per thread
-};
-
 // Slots whose gathers a thread issues together in rows of eight and more: all
 // of them where latency counts, four in the deep form (registers: the batch of
 // eight made A^T at n = 20 with 19 instances 213 us instead of 151).
 __host__ __device__ constexpr int wide_batch(bool deep) { return deep ? 4 : 8; }
-
-// Rows per thread of the deep form, by bucket width.
-__host__ __device__ constexpr int ell_depth(int W) { return W == 1 ? 4 : (W == 2 ? 2 : 1); }
 
 // One thread's place among the tiles of a bucket.
 struct Lane {
@@ -411,7 +397,7 @@ template <int WB, int MODE, bool DEEP, bool STREAM, bool PK, bool COH, class Epi
 __device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int nbatch, int t0, int tstep, Lane& L,
                                          const double* __restrict__ in, const Epi& e, const double* sbook,
                                          double (&dot)[2]) {
-    constexpr int R = DEEP ? ell_depth(WB) : 1;
+    constexpr int R = unit_passes(DEEP, WB);
     constexpr bool WIDE = WB == wide_batch(DEEP);  // also the bucket of four in the deep form, with one batch
     constexpr int32_t kCol = PK ? (1 << kCodeShift) - 1 : -1;
     static_assert(!DEEP || PK, "the deep form reads packed tables");
@@ -617,12 +603,8 @@ __device__ __forceinline__ double ell_cta(const DevMap& M, const Blocks& bl, int
     if (L.rsub < L.rpp && (L.on0 || L.on1)) {
 #pragma unroll 1
         for (int bi = 0; bi < M.nb; bi++) {
-            // the first unit of this bucket that is this CTA's
-            int t0 = (int)blockIdx.x - bl.start[bi];
-            if (t0 < 0) {
-                if (G >= bl.start[kMaxBuckets]) break;  // one unit per CTA
-                t0 = (t0 % G + G) % G;
-            }
+            const int t0 = first_tile(bl, bi, (int)blockIdx.x, G);
+            if (t0 < 0) break;
             if (t0 >= bl.start[bi + 1] - bl.start[bi]) continue;
             const int W = M.width[bi];
             if (W == 1)
@@ -1313,44 +1295,13 @@ static bool map_streamed(const DevMap& M, int B) {
     return B >= 8;
 }
 
-// CTA size for B instances: whole passes of a row's lanes, rounded up to
-// warps, and at least B (the per-instance sums end in thread b < B).
-static int map_threads(int B) {
-    const int n = lanes_of(B);
-    return std::max(kThreads / n * n, B) + 31 & ~31;
-}
-
-// Units of a map (Blocks).  Small maps (at most deep_from tiles with one row per
-// thread, as many as are resident at once) keep one row per thread: there the
-// kernel is one latency chain, and more CTAs spread it wider.
-static Blocks map_blocks(const DevMap& M, int B, int threads, int deep_from) {
-    Blocks bl{};
-    const int64_t rpp = threads / lanes_of(B);
-    auto tiles = [&](int i, bool deep) {
-        const int64_t per = rpp * (deep ? ell_depth(M.width[i]) : 1);
-        return (M.nslots[i] + per - 1) / per;
-    };
-    int64_t tot = 0;
-    for (int i = 0; i < M.nb; i++) tot += tiles(i, false);
-    bl.deep = M.packed && tot > deep_from;
-    bl.mid = M.nlong - M.nmid;
-    bl.midchunks = (B + 31) / 32;
-    const int warps = threads / 32;
-    int acc = bl.mid + (M.nmid + warps - 1) / warps * bl.midchunks;
-    for (int i = 0; i < M.nb; i++) {
-        bl.start[i] = acc;
-        acc += (int)tiles(i, bl.deep != 0);
-    }
-    for (int i = M.nb; i <= kMaxBuckets; i++) bl.start[i] = acc;
-    return bl;
-}
-
 // Returns the partial sums written per instance (one per CTA, where the
 // epilogue sums).
 template <class Epi>
 static int run_map(const DevMap& M, int B, const double* in, const Epi& e, double* partial, cudaStream_t s) {
     const int threads = map_threads(B);
-    const Blocks bl = map_blocks(M, B, threads, 148 * kMapCtasPerSm);
+    const bool deep = wants_deep(M, B, threads, 148 * kMapCtasPerSm);
+    const Blocks bl = map_blocks(M, B, threads, deep);
     const int units = bl.start[kMaxBuckets];
     if (units == 0) return 0;
     // as many CTAs as fit on the device at once, each with its share of the units
@@ -1358,9 +1309,9 @@ static int run_map(const DevMap& M, int B, const double* in, const Epi& e, doubl
     const bool st = map_streamed(M, B);
     auto go = [&](auto mode) {
         constexpr int MODE = decltype(mode)::value;
-        auto k = bl.deep ? (st ? ell_kernel<MODE, true, true, true, Epi> : ell_kernel<MODE, true, false, true, Epi>)
-                         : (M.packed ? ell_kernel<MODE, false, false, true, Epi>
-                                     : ell_kernel<MODE, false, false, false, Epi>);
+        auto k = deep ? (st ? ell_kernel<MODE, true, true, true, Epi> : ell_kernel<MODE, true, false, true, Epi>)
+                      : (M.packed ? ell_kernel<MODE, false, false, true, Epi>
+                                  : ell_kernel<MODE, false, false, false, Epi>);
         cudaLaunchAttribute attr{};
         attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr.val.programmaticStreamSerializationAllowed = 1;
@@ -1585,8 +1536,9 @@ cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, const doubl
     CgLoopArgs L;
     L.A = A;
     L.AT = AT;
-    L.blA = map_blocks(L.A, B, kLoopThreads, 4 * grid);
-    L.blAT = map_blocks(L.AT, B, kLoopThreads, 4 * grid);
+    const LoopUnits units = loop_units(A, AT, B, kLoopThreads, 4 * grid);
+    L.blA = units.A;
+    L.blAT = units.AT;
     // no more CTAs than the larger map has units: a barrier costs by its CTAs
     grid = std::min(grid, std::max(L.blA.start[kMaxBuckets], L.blAT.start[kMaxBuckets]));
     L.B = B;
@@ -1607,8 +1559,8 @@ cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, const doubl
     auto pick = [&](auto mode) -> const void* {
         constexpr int MODE = decltype(mode)::value;
         if (!A.packed || !AT.packed) return (const void*)cg_loop_kernel<MODE, false, false>;
-        return L.blA.deep && L.blAT.deep ? (const void*)cg_loop_kernel<MODE, true, true>
-                                         : (const void*)cg_loop_kernel<MODE, false, true>;
+        return units.deep ? (const void*)cg_loop_kernel<MODE, true, true>
+                          : (const void*)cg_loop_kernel<MODE, false, true>;
     };
     const LaneMode lm = lane_mode(B);
     const void* fn = lm == kOne ? pick(std::integral_constant<int, kOne>())

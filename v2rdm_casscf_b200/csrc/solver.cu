@@ -191,15 +191,11 @@ struct MapTable {
     }
 
     void build(const Csr& M) {
-        static const int widths[kMaxBuckets] = {1, 2, 4, 5, 8, 16, 32};
         std::vector<std::vector<int32_t>> brow(kMaxBuckets);
         std::vector<int32_t> lrows, lptr(1, 0), lcol;
         std::vector<double> lval;
         for (int64_t r = 0; r < M.nrows; r++) {
-            const int64_t len = M.rowptr[r + 1] - M.rowptr[r];
-            int w = 0;
-            while (w < kMaxBuckets && widths[w] < len) w++;
-            if (M.nrows < kLatencyRows && len > 16) w = kMaxBuckets;
+            const int w = row_bucket(M.nrows, M.rowptr[r + 1] - M.rowptr[r]);
             if (w < kMaxBuckets) {
                 brow[w].push_back((int32_t)r);
             } else {
@@ -214,7 +210,7 @@ struct MapTable {
         for (int32_t r : lrows) same[M.rowptr[r + 1] - M.rowptr[r]]++;
         const auto mid_end = std::stable_partition(lrows.begin(), lrows.end(), [&](int32_t r) {
             const int64_t len = M.rowptr[r + 1] - M.rowptr[r];
-            return len <= kMidRow && (same[len] >= kMidMany || len <= 32);
+            return row_is_mid(len, same[len]);
         });
         for (int32_t r : lrows) {
             for (int64_t k = M.rowptr[r]; k < M.rowptr[r + 1]; k++) {
@@ -238,7 +234,7 @@ struct MapTable {
         dm.nrows = M.nrows;
         for (int w = 0; w < kMaxBuckets; w++) {
             if (brow[w].empty()) continue;
-            const int W = widths[w];
+            const int W = kBucketWidths[w];
             const int64_t ns = (int64_t)brow[w].size();
             const int bi = dm.nb++;
             dm.width[bi] = W;
