@@ -80,8 +80,9 @@ static long faults(const Map& M, const Blocks& bl, int B, int threads, int G, bo
     return bad;
 }
 
-int main() {
+int main(int argc, char**) {
     const Map A = read_map(), AT = read_map();
+    if (argc > 1) return loop_applies(A, AT) ? 0 : 2;
     for (int B = 1; B <= 40; B++) {
         const int t = map_threads(B);
         for (const Map* M : {&A, &AT}) {
@@ -130,3 +131,10 @@ def test_every_row_has_one_unit(v2g, driver, n, positivity, spin, mixed):
     rows = [r.split() for r in out.splitlines()]
     assert {int(b) for kind, b, v in rows if kind == "mixed" and int(v)} >= set(mixed)
     assert [r for r in rows if r[0] != "mixed" and int(r[2])] == []
+
+
+@pytest.mark.parametrize("packed", [(0, 0), (0, 1), (1, 0), (1, 1)])
+def test_one_kernel_for_both_maps_needs_one_packing(driver, packed):
+    data = b"".join(np.array([3, p], dtype=np.int64).tobytes() + np.array([1, 2, 3], dtype=np.int32).tobytes()
+                    for p in packed)
+    assert (subprocess.run([driver, "applies"], input=data).returncode == 0) == (packed[0] == packed[1])

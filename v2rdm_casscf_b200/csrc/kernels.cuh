@@ -137,7 +137,7 @@ void launch_cg_while(cudaGraphConditionalHandle h, const int* n_active, int* cou
 // n = 20 one instance 131 / 99).
 constexpr int kLoopMaxB = 8;
 constexpr int64_t kLoopMaxRows = 300000;
-bool cg_loop_fits(int64_t nc, int B);
+bool cg_loop_fits(const DevMap& A, const DevMap& AT, int B);
 // CTAs of the cooperative grid on this device (0: no cooperative launch)
 int cg_loop_grid(int device);
 size_t cg_loop_slots(int grid, int B);

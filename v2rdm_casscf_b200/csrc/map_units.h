@@ -103,6 +103,12 @@ Blocks map_blocks(const Map& M, int B, int threads, bool deep) {
 
 // The units of A and A^T for one kernel that applies both (the persistent CG):
 // one form for the two maps, deep only where both ask for it.
+// The tables have to be both packed or both not, since one kernel reads both (each
+// table is packed by its own coefficients).
+template <class Map>
+bool loop_applies(const Map& A, const Map& AT) {
+    return (A.packed != 0) == (AT.packed != 0);
+}
 struct LoopUnits {
     bool deep;
     Blocks A, AT;

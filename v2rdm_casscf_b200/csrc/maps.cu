@@ -1474,7 +1474,9 @@ int cg_loop_grid(int device) {
 
 size_t cg_loop_slots(int grid, int B) { return 3 * (size_t)grid * B * kSlotStride; }
 
-bool cg_loop_fits(int64_t nc, int B) { return B >= 1 && B <= kLoopMaxB && nc <= kLoopMaxRows; }
+bool cg_loop_fits(const DevMap& A, const DevMap& AT, int B) {
+    return B >= 1 && B <= kLoopMaxB && A.nrows <= kLoopMaxRows && loop_applies(A, AT);
+}
 
 // The rows of M dealt to warps for B instances; false when they do not fit
 // (unpacked, or rows longer than 8 entries for each of 32 / B lanes).
@@ -1558,7 +1560,7 @@ cudaError_t launch_cg_loop(const DevMap& A, const DevMap& AT, int B, const doubl
     void* args[] = {&L};
     auto pick = [&](auto mode) -> const void* {
         constexpr int MODE = decltype(mode)::value;
-        if (!A.packed || !AT.packed) return (const void*)cg_loop_kernel<MODE, false, false>;
+        if (!A.packed) return (const void*)cg_loop_kernel<MODE, false, false>;
         return units.deep ? (const void*)cg_loop_kernel<MODE, true, true>
                           : (const void*)cg_loop_kernel<MODE, false, true>;
     };

@@ -427,7 +427,7 @@ class GroupRun {
         hcs_buf_.alloc(B_);
         hcs_ = hcs_buf_.p;
         tune_maps();
-        if (cg_loop_fits(nc_, B_)) loop_grid_ = cg_loop_grid(T.device);
+        if (cg_loop_fits(mA_, mAT_, B_)) loop_grid_ = cg_loop_grid(T.device);
         if (loop_grid_ > 0) {
             looperr_.alloc(1);
             loopslots_.alloc(cg_loop_slots(loop_grid_, B_));
