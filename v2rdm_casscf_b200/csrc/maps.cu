@@ -171,7 +171,10 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 // Predicated loads without a branch around each (the compiler's form of a
 // conditional load costs more instructions than the load): p where ok, else
-// the default (-1, 0).  COH: through L2 (ld.global.cg), for vectors that other
+// the default (-1, 0).  Table loads (load_word, load_val) are read-only loads that
+// the compiler may place before pdl_wait; vectors, which the previous kernel of
+// the stream may still be writing until then, are read by load_one and load_two,
+// ordered after the wait.  COH: through L2 (ld.global.cg), for vectors that other
 // CTAs of the same (persistent) launch write, never from a stale L1 line.
 template <bool STREAM>
 __device__ __forceinline__ int32_t load_word(const int32_t* p, bool ok) {
@@ -186,6 +189,14 @@ __device__ __forceinline__ int32_t load_word(const int32_t* p, bool ok) {
             : "l"(p), "r"((int)ok));
     return v;
 }
+__device__ __forceinline__ double load_val(const double* p, bool ok) {
+    double v;
+    asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+        "@q ld.global.nc.f64 %0, [%1];\n\t}"
+        : "=&d"(v)
+        : "l"(p), "r"((int)ok));
+    return v;
+}
 template <bool COH>
 __device__ __forceinline__ double load_one(const double* p, bool ok) {
     double v;
@@ -197,10 +208,21 @@ __device__ __forceinline__ double load_one(const double* p, bool ok) {
             : "l"(p), "r"((int)ok)
             : "memory");
     else
-        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
-            "@q ld.global.nc.f64 %0, [%1];\n\t}"
+        asm volatile(
+            "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+            "@q ld.global.f64 %0, [%1];\n\t}"
             : "=&d"(v)
-            : "l"(p), "r"((int)ok));
+            : "l"(p), "r"((int)ok)
+            : "memory");
+    return v;
+}
+template <bool COH>
+__device__ __forceinline__ double load_one(const double* p) {
+    double v;
+    if (COH)
+        asm volatile("ld.global.cg.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+    else
+        asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
 template <bool COH>
@@ -214,10 +236,12 @@ __device__ __forceinline__ double2 load_two(const double* p, bool ok) {
             : "l"(p), "r"((int)ok)
             : "memory");
     else
-        asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
-            "mov.f64 %1, 0d0000000000000000;\n\t@q ld.global.nc.v2.f64 {%0, %1}, [%2];\n\t}"
+        asm volatile(
+            "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.f64 %0, 0d0000000000000000;\n\t"
+            "mov.f64 %1, 0d0000000000000000;\n\t@q ld.global.v2.f64 {%0, %1}, [%2];\n\t}"
             : "=&d"(v.x), "=&d"(v.y)
-            : "l"(p), "r"((int)ok));
+            : "l"(p), "r"((int)ok)
+            : "memory");
     return v;
 }
 
@@ -395,7 +419,7 @@ struct EpiCgInit {
 // doubles a row), so table offsets are 32-bit.
 template <int WB, int MODE, bool DEEP, bool STREAM, bool PK, bool COH, class Epi>
 __device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int nbatch, int t0, int tstep, Lane& L,
-                                         const double* __restrict__ in, const Epi& e, const double* sbook,
+                                         const double* in, const Epi& e, const double* sbook,
                                          double (&dot)[2]) {
     constexpr int R = unit_passes(DEEP, WB);
     constexpr bool WIDE = WB == wide_batch(DEEP);  // also the bucket of four in the deep form, with one batch
@@ -463,7 +487,7 @@ __device__ __forceinline__ void ell_rows(const DevMap& M, int bi, int nbatch, in
                                 ok && L.b1 < L.B);
                     }
                     if (!PK)
-                        v[k][j] = load_one<false>(vals + (size_t)((kb * WB + k) * ns + (uint32_t)i + j * rpp), ok);
+                        v[k][j] = load_val(vals + (size_t)((kb * WB + k) * ns + (uint32_t)i + j * rpp), ok);
                 }
             int32_t wn[WB][R];
             if (WIDE && kb + 1 < nbatch) {
@@ -522,7 +546,7 @@ __device__ __forceinline__ double warps_to_instances(double v, int c0, int cnt) 
 // (the long form) left the 5,792 such rows of A^T at n = 8 with T2 with 80
 // entries on 256 threads each (38 us of a 48 us launch at one instance).
 template <bool COH, class Epi>
-__device__ __forceinline__ double mid_rows(const DevMap& M, int B, const double* __restrict__ in, const Epi& e,
+__device__ __forceinline__ double mid_rows(const DevMap& M, int B, const double* in, const Epi& e,
                                            int group, int chunk) {
     const int lane = threadIdx.x & 31;
     const int m = group * (int)(blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -536,7 +560,7 @@ __device__ __forceinline__ double mid_rows(const DevMap& M, int B, const double*
 #pragma unroll 8
             for (int k = k0 + l; k < k1; k += n) {
                 const double* g = in + (int64_t)__ldg(M.long_col + k) * B + b;
-                s += __ldg(M.long_val + k) * (COH ? __ldcg(g) : __ldg(g));
+                s += __ldg(M.long_val + k) * load_one<COH>(g);
             }
         }
         for (int left = n; left > 1;) {
@@ -556,7 +580,7 @@ __device__ __forceinline__ double mid_rows(const DevMap& M, int B, const double*
 // Long rows: one CTA per row; thread t sums entries k = t / B, t / B + T / B,
 // ... for instance t % B, then a fixed-order reduction per instance.
 template <bool COH, class Epi>
-__device__ __forceinline__ double long_row(const DevMap& M, int B, const double* __restrict__ in, const Epi& e,
+__device__ __forceinline__ double long_row(const DevMap& M, int B, const double* in, const Epi& e,
                                            int lr) {
     const int lanes = blockDim.x / B;
     const int b = threadIdx.x % B;
@@ -567,7 +591,7 @@ __device__ __forceinline__ double long_row(const DevMap& M, int B, const double*
 #pragma unroll 4
         for (int k = k0 + l; k < k1; k += lanes) {
             const double* g = in + (int64_t)__ldg(M.long_col + k) * B + b;
-            s += __ldg(M.long_val + k) * (COH ? __ldcg(g) : __ldg(g));
+            s += __ldg(M.long_val + k) * load_one<COH>(g);
         }
     }
     const double t = cta_instance_sum(s, B);
@@ -582,7 +606,7 @@ __device__ __forceinline__ double long_row(const DevMap& M, int B, const double*
 // All the units of this CTA: returns to thread b < B the CTA's sum of the
 // optional dot for instance b (fixed order; 0 elsewhere).
 template <int MODE, bool DEEP, bool STREAM, bool PK, bool COH, class Epi>
-__device__ __forceinline__ double ell_cta(const DevMap& M, const Blocks& bl, int B, const double* __restrict__ in,
+__device__ __forceinline__ double ell_cta(const DevMap& M, const Blocks& bl, int B, const double* in,
                                           const Epi& e, const double* sbook) {
     const int G = (int)gridDim.x;
     double sum = 0.0;  // thread b: instance b
@@ -645,7 +669,7 @@ __device__ __forceinline__ double ell_cta(const DevMap& M, const Blocks& bl, int
 template <int MODE, bool DEEP, bool STREAM, bool PK, class Epi>
 __global__ void __launch_bounds__(kThreads, kMapCtasPerSm)
     ell_kernel(const __grid_constant__ DevMap M, const __grid_constant__ Blocks bl, int B,
-               const double* __restrict__ in, const __grid_constant__ Epi e, double* __restrict__ partial) {
+               const double* in, const __grid_constant__ Epi e, double* __restrict__ partial) {
     pdl_trigger();
     // the coefficient book of a packed table, in shared memory
     __shared__ double sbook[kBookSize];
