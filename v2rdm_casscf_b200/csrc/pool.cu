@@ -46,33 +46,61 @@ size_t pinned_size(size_t bytes) {
 
 }  // namespace
 
+namespace {
+
+// alloc(), once more without what the pool holds unused if that is in the way
+template <class F>
+cudaError_t retried(cudaMemPool_t pool, F&& alloc) {
+    cudaError_t e = alloc();
+    if (e == cudaErrorMemoryAllocation && pool) {
+        cudaGetLastError();
+        cudaStreamSynchronize(cudaStreamLegacy);
+        cudaMemPoolTrimTo(pool, 0);
+        e = alloc();
+    }
+    return e;
+}
+
+template <class F>
+void on_device(int device, F&& f) {
+    int prev = -1;
+    if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
+    if (prev != device) cudaSetDevice(device);
+    f();
+    if (prev >= 0 && prev != device) cudaSetDevice(prev);
+}
+
+}  // namespace
+
 cudaError_t pool_alloc(void** p, size_t bytes) {
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     const cudaMemPool_t pool = pool_of(device);
     if (!pool) return cudaMalloc(p, bytes);
-    e = cudaMallocFromPoolAsync(p, bytes, pool, cudaStreamLegacy);
-    if (e == cudaErrorMemoryAllocation) {
-        // what the pool holds unused may be in the way
-        cudaGetLastError();
-        cudaStreamSynchronize(cudaStreamLegacy);
-        cudaMemPoolTrimTo(pool, 0);
-        e = cudaMallocFromPoolAsync(p, bytes, pool, cudaStreamLegacy);
-    }
-    return e;
+    return retried(pool, [&] { return cudaMallocFromPoolAsync(p, bytes, pool, cudaStreamLegacy); });
 }
 
 void pool_free(void* p, int device) {
     if (!p) return;
-    int prev = -1;
-    if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
-    if (prev != device) cudaSetDevice(device);
-    if (pool_of(device))
-        cudaFreeAsync(p, cudaStreamLegacy);
-    else
-        cudaFree(p);
-    if (prev >= 0 && prev != device) cudaSetDevice(prev);
+    on_device(device, [&] {
+        if (pool_of(device))
+            cudaFreeAsync(p, cudaStreamLegacy);
+        else
+            cudaFree(p);
+    });
+}
+
+cudaError_t device_alloc(void** p, size_t bytes) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    return retried(pool_of(device), [&] { return cudaMalloc(p, bytes); });
+}
+
+void device_free(void* p, int device) {
+    if (!p) return;
+    on_device(device, [&] { cudaFree(p); });
 }
 
 cudaError_t pinned_alloc(void** p, size_t bytes) {

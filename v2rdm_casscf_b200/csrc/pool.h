@@ -26,6 +26,11 @@ constexpr size_t kPinnedKeep = size_t(16) << 20;
 cudaError_t pool_alloc(void** p, size_t bytes);
 void pool_free(void* p, int device);  // device: where it was allocated
 
+// Device memory outside the pool, for what a caller's streams may still read when
+// its owner goes: device_free waits for the device, whatever the stream.
+cudaError_t device_alloc(void** p, size_t bytes);
+void device_free(void* p, int device);
+
 // Page-locked host memory, in powers of two.  Give back only what no copy in
 // flight uses.
 cudaError_t pinned_alloc(void** p, size_t bytes);

@@ -98,6 +98,31 @@ struct DevBuf {
     }
 };
 
+// What a handle's asynchronous entries read: a caller's stream, of which the
+// library keeps nothing, may still be at work on it when the handle goes, so the
+// memory is given back by cudaFree, which waits for the device.  (The pool's frees
+// are ordered by the legacy stream alone; the streams that the other buffers are
+// used on are synchronised by their owners first.)
+template <class T>
+struct TableBuf {
+    T* p = nullptr;
+    int device = 0;
+    TableBuf() = default;
+    TableBuf(const TableBuf&) = delete;
+    TableBuf& operator=(const TableBuf&) = delete;
+    ~TableBuf() { device_free(p, device); }
+    void upload(const T* h, size_t count) {
+        device_free(p, device);
+        p = nullptr;
+        if (!count) return;
+        CK(cudaGetDevice(&device));
+        void* q = nullptr;
+        CK(device_alloc(&q, count * sizeof(T)));
+        p = static_cast<T*>(q);
+        CK(cudaMemcpy(p, h, count * sizeof(T), cudaMemcpyHostToDevice));
+    }
+};
+
 // Page-locked host memory for copies on the streams of its owner.
 template <class T>
 struct HostBuf {
@@ -118,10 +143,12 @@ struct HostBuf {
     }
 };
 
-// One map (A or A^T) on the device in the bucketed-ELL form of kernels.cuh.
+// One map (A or A^T) on the device in the bucketed-ELL form of kernels.cuh, in
+// TableBuf (a handle's) or DevBuf (used and dropped inside one call).
+template <template <class> class Buf>
 struct MapTable {
-    DevBuf<int32_t> rows, cols, long_rows, long_ptr, long_col, res_row, res_ptr, res_word;
-    DevBuf<double> vals, long_val;
+    Buf<int32_t> rows, cols, long_rows, long_ptr, long_col, res_row, res_ptr, res_word;
+    Buf<double> vals, long_val;
     DevMap dm;
 
     // Packs the coefficient of every ELL entry into its column word when the
@@ -283,8 +310,8 @@ struct DeviceTables {
     Layout L;
     int device = 0;
     Csr hA;  // kept on the host for v2g_export_A
-    MapTable mA, mAT;
-    DevBuf<double> b;
+    MapTable<TableBuf> mA, mAT;
+    TableBuf<double> b;
     std::vector<double> hb;
     const DevMap& A() const { return mA.dm; }
     const DevMap& AT() const { return mAT.dm; }
@@ -2066,7 +2093,7 @@ int v2g_pack_spatial_density(v2g_handle* h, const double* active_energies, doubl
         v2g::build_spatial_map(P.L, active_energies ? active_energies : (P.energies.empty() ? nullptr : P.energies.data()),
                                M, n1, n2);
         CK(cudaSetDevice(P.device));
-        v2g::MapTable T;
+        v2g::MapTable<v2g::DevBuf> T;
         T.build(M);
         v2g::DevBuf<double> x, out;
         x.upload(P.x.data(), P.x.size());
