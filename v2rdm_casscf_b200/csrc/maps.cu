@@ -110,8 +110,9 @@ constexpr int kLoopThreads = 512;  // CTA of the persistent CG
 constexpr int kWarps = 32;         // of the largest CTA
 
 // How instances map to lanes: one lane each (B = 1), or two instances per
-// lane: l and l + (B + 1) / 2 for odd B (contiguous 8-byte loads), 2 l and
-// 2 l + 1 for even B (16-byte loads).
+// lane: l and l + (B + 1) / 2 (contiguous 8-byte loads) for odd B, and for even B
+// where the input is not on a 16-byte boundary; 2 l and 2 l + 1 (16-byte loads)
+// for even B else.
 enum LaneMode { kOne = 0, kOdd = 1, kEven = 2 };
 static LaneMode lane_mode(int B) { return B == 1 ? kOne : ((B & 1) ? kOdd : kEven); }
 
@@ -1331,6 +1332,7 @@ static int run_map(const DevMap& M, int B, const double* in, const Epi& e, doubl
     // as many CTAs as fit on the device at once, each with its share of the units
     const int g = std::min(units, 148 * kMapCtasPerSm);
     const bool st = map_streamed(M, B);
+    const LaneMode mode = lane_mode(B) == kEven && ((uintptr_t)in & 15) != 0 ? kOdd : lane_mode(B);
     auto go = [&](auto mode) {
         constexpr int MODE = decltype(mode)::value;
         auto k = deep ? (st ? ell_kernel<MODE, true, true, true, Epi> : ell_kernel<MODE, true, false, true, Epi>)
@@ -1347,7 +1349,7 @@ static int run_map(const DevMap& M, int B, const double* in, const Epi& e, doubl
         cfg.numAttrs = 1;
         cudaLaunchKernelEx(&cfg, k, M, bl, B, in, e, partial);
     };
-    switch (lane_mode(B)) {
+    switch (mode) {
         case kOne: go(std::integral_constant<int, kOne>()); break;
         case kOdd: go(std::integral_constant<int, kOdd>()); break;
         default: go(std::integral_constant<int, kEven>()); break;
