@@ -300,6 +300,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const BlockTask* __
     if (ok) {
         const int row = m0 + warp * 32 + lane;
         const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16);
+        const bool wide = ((uintptr_t)C & 15) == 0;  // a caller's C may start on any 8-byte boundary
 #pragma unroll 1
         for (int h = 0; h < kTcN / 32; h++) {
             float v[32];
@@ -307,8 +308,14 @@ __global__ void __launch_bounds__(kTcThreads) tc_gemm_kernel(const BlockTask* __
             const int col0 = n0 + h * 32;
             if (row < np && col0 < np) {
                 double* o = c + (int64_t)row * np + col0;
+                if (wide) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 2) *reinterpret_cast<double2*>(o + j) = make_double2((double)v[j], (double)v[j + 1]);
+                    for (int j = 0; j < 32; j += 2)
+                        *reinterpret_cast<double2*>(o + j) = make_double2((double)v[j], (double)v[j + 1]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 32; j++) o[j] = (double)v[j];
+                }
             }
         }
     }
