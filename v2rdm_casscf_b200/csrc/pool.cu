@@ -84,10 +84,8 @@ cudaError_t pool_alloc(void** p, size_t bytes) {
 void pool_free(void* p, int device) {
     if (!p) return;
     on_device(device, [&] {
-        if (pool_of(device))
-            cudaFreeAsync(p, cudaStreamLegacy);
-        else
-            cudaFree(p);
+        // refused where a caller's own capture forbids work on the legacy stream
+        if (!pool_of(device) || cudaFreeAsync(p, cudaStreamLegacy) != cudaSuccess) cudaFree(p);
     });
 }
 

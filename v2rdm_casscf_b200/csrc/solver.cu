@@ -1301,14 +1301,34 @@ class GroupRun {
         timed(mAT_, [&] { launch_cg_direction(mAT_, B_, r_.p, atp_.p, cs_.p, partial_.p, nact_.p, s_); });
         timed(mA_, [&] { launch_cg_step(mA_, B_, atp_.p, y_.p, r_.p, p_.p, cs_.p, partial_.p, nact_.p, s_); });
     }
-    // kCgChunk CG iterations captured from the stream into a graph: the
+    // Captures take a non-blocking stream of their own in place of s_.  The group's
+    // streams wait for the legacy default stream and it for them: while one of
+    // them captured, an allocation, copy or free on the legacy stream in another
+    // thread would be refused and end the capture.
+    struct CaptureStream {
+        cudaStream_t &s, own = nullptr, saved;
+        explicit CaptureStream(cudaStream_t& stream) : s(stream), saved(stream) {
+            CK(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+            s = own;
+        }
+        CaptureStream(const CaptureStream&) = delete;
+        CaptureStream& operator=(const CaptureStream&) = delete;
+        ~CaptureStream() {
+            s = saved;
+            cudaStreamDestroy(own);
+        }
+    };
+    // kCgChunk CG iterations captured from a stream into a graph: the
     // kernels' arguments are the group's fixed buffers, so one capture serves
     // every CG solve of the group.
     void capture_cg_chunk() {
-        CK(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
-        for (int k = 0; k < kCgChunk; k++) cg_iteration();
         cudaGraph_t g = nullptr;
-        CK(cudaStreamEndCapture(s_, &g));
+        {
+            CaptureStream cap(s_);
+            CK(cudaStreamBeginCapture(s_, cudaStreamCaptureModeThreadLocal));
+            for (int k = 0; k < kCgChunk; k++) cg_iteration();
+            CK(cudaStreamEndCapture(s_, &g));
+        }
         size_t nodes = 0;
         CK(cudaGraphGetNodes(g, nullptr, &nodes));
         // the launchers counted the captured kernels as launches; graph
@@ -1349,11 +1369,15 @@ class GroupRun {
             return;
         }
         cudaGraph_t body = cp.conditional.phGraph_out[0];
-        CK(cudaStreamBeginCaptureToGraph(s_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        cg_iteration();
-        launch_cg_while(h, nact_.p, nact_.p + 6, cap, s_);
-        cudaGraph_t captured = nullptr;
-        const cudaError_t ce = cudaStreamEndCapture(s_, &captured);
+        cudaError_t ce;
+        {
+            CaptureStream own(s_);
+            CK(cudaStreamBeginCaptureToGraph(s_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+            cg_iteration();
+            launch_cg_while(h, nact_.p, nact_.p + 6, cap, s_);
+            cudaGraph_t captured = nullptr;
+            ce = cudaStreamEndCapture(s_, &captured);
+        }
         size_t nodes = 0;
         if (ce == cudaSuccess) cudaGraphGetNodes(body, nullptr, &nodes);
         // the launchers counted the captured kernels; replays are counted per iteration
@@ -2159,7 +2183,9 @@ int v2g_solve_batch(v2g_handle** hs, int count, v2g_result* res) {
                 members.push_back(which);
             }
         }
-        CK(cudaDeviceSynchronize());
+        // (the legacy stream waits for the groups' streams; a synchronisation of the
+        // device would be refused while another thread's solve captures its graph)
+        CK(cudaStreamSynchronize(0));
         CK(cudaEventRecord(t1, 0));
         const long launches0 = v2g::g_kernel_launches.load();
         // every layout group runs its own lock-step loop on its own stream
@@ -2178,7 +2204,7 @@ int v2g_solve_batch(v2g_handle** hs, int count, v2g_result* res) {
         for (auto& t : th) t.join();
         for (auto& e : errs)
             if (!e.empty()) throw v2g::CudaError(e);
-        CK(cudaDeviceSynchronize());
+        CK(cudaStreamSynchronize(0));
         CK(cudaEventRecord(t2, 0));
         const long launches1 = v2g::g_kernel_launches.load();
         for (auto& r : runs) r->download_state();
