@@ -1010,8 +1010,9 @@ class GroupRun {
     // V2G_DIAG_FILE or stderr): per instance eps(p), eps(d), mu, this
     // iteration's CG count, |y|^2, |x|^2, |z|^2; per group the largest distance
     // of the projection's eigenvectors from orthonormal (max |V^T V - I| over the
-    // large blocks, as the refinement found it) and the running counts of
-    // block-Jacobi fallbacks and cold restarts.
+    // large blocks, as the refinement found it; 0 for groups projected by the
+    // matrix sign, which keep none) and the running counts of block-Jacobi
+    // fallbacks and cold restarts.
     void diagnose(int it, const std::vector<CgScalars>& cs, const std::vector<double>& ep,
                   const std::vector<double>& ed, const std::vector<double>& mu) {
         std::vector<double> sums(3 * B_);
@@ -1022,7 +1023,7 @@ class GroupRun {
             CK(cudaMemcpyAsync(&sums[k * B_], red_.p, B_ * sizeof(double), cudaMemcpyDeviceToHost, s_));
         }
         double gmax = 0.0;
-        if (nlarge_ > 0) {
+        if (nlarge_ > 0 && sign_grid_ == 0) {
             std::vector<unsigned long long> g(nlarge_);
             CK(cudaMemcpyAsync(g.data(), gdev_.p, nlarge_ * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s_));
             CK(cudaStreamSynchronize(s_));
