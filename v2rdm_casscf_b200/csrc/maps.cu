@@ -12,6 +12,7 @@
 #include <type_traits>
 
 #include "kernels.cuh"
+#include "wait.cuh"
 
 namespace v2g {
 
@@ -995,11 +996,9 @@ __global__ void cg_reduce_kernel(int what, int nblk, int B, const double* __rest
 // exchanges and the latency of the gathers (the vectors sit in L2).  Every CTA
 // adds the posted sums itself in the same fixed order, so every CTA holds the same scalars and takes the same decision to continue; no CTA
 // waits for a value only another CTA computes.  Vectors written inside the
-// launch are read through L2 (ld.global.cg).  Each barrier wait is bounded: a
-// wait that runs out sets *err and the CTA leaves the kernel; the others then
-// run out at their next wait.
-
-constexpr long kGridWaitPolls = 1L << 25;  // about a second of polling (short sleeps)
+// launch are read through L2 (ld.global.cg).  Each barrier wait is bounded
+// (wait.cuh): a wait that runs out sets *err and the CTA leaves the kernel; the
+// others see *err in theirs and leave too.
 
 struct CgLoopArgs {
     DevMap A, AT;
@@ -1049,12 +1048,13 @@ __device__ __forceinline__ bool grid_exchange(unsigned long long* sets, unsigned
     bool fine = true;
     if (t < lanes) {
         long polls = 0;
+        unsigned long long start = 0;
         for (int k = t; k < n && fine; k += lanes) {
             unsigned long long bits;
             while (true) {
                 asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(bits) : "l"(S + (size_t)k * kSlotStride) : "memory");
                 if (bits != kSlotEmpty) break;
-                if (++polls >= kGridWaitPolls) {
+                if (wait_is_over(polls++, start, err)) {
                     atomicExch(err, 1);
                     fine = false;
                     break;

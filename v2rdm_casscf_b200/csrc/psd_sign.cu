@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "wait.cuh"
 
 namespace v2g {
 
@@ -304,7 +305,6 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS == kSmallWarps ? 1 : 2)
 constexpr int kTeamThreads = 256;
 constexpr int kTile = 32, kChunkLd = kTile + 4, kRing = 4;
 constexpr int kChunk = kTile * kChunkLd;  // one operand's chunk in shared memory
-constexpr long kTeamPolls = 1L << 25;     // about a second of polling (short sleeps)
 
 // All CTAs of the team have arrived `target / size` times; false when the wait ran out.
 __device__ __forceinline__ bool team_wait(unsigned int* bar, unsigned int target, int* err) {
@@ -314,10 +314,11 @@ __device__ __forceinline__ bool team_wait(unsigned int* bar, unsigned int target
         ok = 1;
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         unsigned int v = 0;
+        unsigned long long start = 0;
         for (long n = 0;; n++) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
             if (v >= target) break;
-            if (n >= kTeamPolls) {
+            if (wait_is_over(n, start, err)) {
                 atomicExch(err, 1);
                 ok = 0;
                 break;
