@@ -111,7 +111,7 @@ struct TableBuf {
     TableBuf(const TableBuf&) = delete;
     TableBuf& operator=(const TableBuf&) = delete;
     ~TableBuf() { device_free(p, device); }
-    void upload(const T* h, size_t count) {
+    void alloc(size_t count, bool) {
         device_free(p, device);
         p = nullptr;
         if (!count) return;
@@ -119,7 +119,10 @@ struct TableBuf {
         void* q = nullptr;
         CK(device_alloc(&q, count * sizeof(T)));
         p = static_cast<T*>(q);
-        CK(cudaMemcpy(p, h, count * sizeof(T), cudaMemcpyHostToDevice));
+    }
+    void upload(const T* h, size_t count) {
+        alloc(count, false);
+        if (count) CK(cudaMemcpy(p, h, count * sizeof(T), cudaMemcpyHostToDevice));
     }
 };
 
@@ -144,12 +147,28 @@ struct HostBuf {
 };
 
 // One map (A or A^T) on the device in the bucketed-ELL form of kernels.cuh, in
-// TableBuf (a handle's) or DevBuf (used and dropped inside one call).
+// one TableBuf (a handle's) or DevBuf (used and dropped inside one call): an
+// allocation per array took 0.2 ms of setting up a small layout.
 template <template <class> class Buf>
 struct MapTable {
-    Buf<int32_t> rows, cols, long_rows, long_ptr, long_col, res_row, res_ptr, res_word;
-    Buf<double> vals, long_val;
+    Buf<char> mem;
     DevMap dm;
+
+    // The arrays of a table side by side in mem, each on a 256-byte boundary: room()
+    // for all of them, then place() in the same order.
+    size_t used = 0;
+    template <class T>
+    void room(const std::vector<T>& v) {
+        used += (v.size() * sizeof(T) + 255) & ~(size_t)255;
+    }
+    template <class T>
+    const T* place(const std::vector<T>& v) {
+        if (v.empty()) return nullptr;
+        char* at = mem.p + used;
+        room(v);
+        CK(cudaMemcpy(at, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+        return reinterpret_cast<const T*>(at);
+    }
 
     // Packs the coefficient of every ELL entry into its column word when the
     // columns fit in kCodeShift bits and the table has at most kBookSize
@@ -182,24 +201,25 @@ struct MapTable {
     // The long rows for the resident CG: sorted by length, entries packed with
     // the same book, which takes up their coefficients too; left out when the
     // book or the 256 entries of a row do not hold them.
-    void pack_long(const Csr& M, std::vector<int32_t> order, std::map<uint64_t, int>& code, std::vector<double>& bk) {
-        int used = (int)code.size();
+    bool pack_long(const Csr& M, std::vector<int32_t>& order, std::vector<int32_t>& ptr, std::vector<int32_t>& word,
+                   std::map<uint64_t, int>& code, std::vector<double>& bk) {
+        int codes = (int)code.size();
         std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
             return M.rowptr[a + 1] - M.rowptr[a] < M.rowptr[b + 1] - M.rowptr[b];
         });
-        std::vector<int32_t> ptr(1, 0), word;
+        ptr.assign(1, 0);
         for (int32_t r : order) {
-            if (M.rowptr[r + 1] - M.rowptr[r] > 256) return;
+            if (M.rowptr[r + 1] - M.rowptr[r] > 256) return false;
             for (int64_t k = M.rowptr[r]; k < M.rowptr[r + 1]; k++) {
                 uint64_t bits;
                 std::memcpy(&bits, &M.val[k], sizeof bits);
                 auto it = code.find(bits);
                 if (it == code.end()) {
-                    if (used == kBookSize) return;
-                    bk[used] = M.val[k];
-                    it = code.emplace(bits, used++).first;
+                    if (codes == kBookSize) return false;
+                    bk[codes] = M.val[k];
+                    it = code.emplace(bits, codes++).first;
                 }
-                if (M.col[k] >= (1 << kCodeShift)) return;
+                if (M.col[k] >= (1 << kCodeShift)) return false;
                 word.push_back(M.col[k] | it->second << kCodeShift);
             }
             ptr.push_back((int32_t)word.size());
@@ -209,12 +229,7 @@ struct MapTable {
             while (at < dm.nres && M.rowptr[order[at] + 1] - M.rowptr[order[at]] <= (16 << c)) at++;
             dm.res_upto[c] = at;
         }
-        res_row.upload(order.data(), order.size());
-        res_ptr.upload(ptr.data(), ptr.size());
-        res_word.upload(word.data(), word.size());
-        dm.res_row = res_row.p;
-        dm.res_ptr = res_ptr.p;
-        dm.res_word = res_word.p;
+        return true;
     }
 
     void build(const Csr& M) {
@@ -283,25 +298,32 @@ struct MapTable {
         }
         std::map<uint64_t, int> code;
         std::vector<double> bk = pack(hcols, hvals, code);
-        rows.upload(hrows.data(), hrows.size());
-        cols.upload(hcols.data(), hcols.size());
-        if (bk.empty()) vals.upload(hvals.data(), hvals.size());
-        if (!bk.empty()) pack_long(M, lrows, code, bk);
-        long_rows.upload(lrows.data(), lrows.size());
-        long_ptr.upload(lptr.data(), lptr.size());
-        long_col.upload(lcol.data(), lcol.size());
-        long_val.upload(lval.data(), lval.size());
-        dm.rows = rows.p;
-        dm.cols = cols.p;
-        dm.vals = bk.empty() ? vals.p : nullptr;
+        if (!bk.empty()) hvals.clear();
+        std::vector<int32_t> res_row = lrows, res_ptr, res_word;
+        if (bk.empty() || !pack_long(M, res_row, res_ptr, res_word, code, bk)) {
+            res_row.clear();
+            res_ptr.clear();
+            res_word.clear();
+        }
+        used = 0;
+        room(hrows), room(hcols), room(hvals), room(lrows), room(lptr), room(lcol), room(lval);
+        room(res_row), room(res_ptr), room(res_word);
+        mem.alloc(used, false);
+        used = 0;
+        dm.rows = place(hrows);
+        dm.cols = place(hcols);
+        dm.vals = place(hvals);
+        dm.long_rows = place(lrows);
+        dm.long_ptr = place(lptr);
+        dm.long_col = place(lcol);
+        dm.long_val = place(lval);
+        dm.res_row = place(res_row);
+        dm.res_ptr = place(res_ptr);
+        dm.res_word = place(res_word);
         dm.packed = !bk.empty();
         std::copy(bk.begin(), bk.end(), dm.book);
         dm.nlong = (int)lrows.size();
         dm.nmid = (int)(mid_end - lrows.begin());
-        dm.long_rows = long_rows.p;
-        dm.long_ptr = long_ptr.p;
-        dm.long_col = long_col.p;
-        dm.long_val = long_val.p;
     }
 };
 
