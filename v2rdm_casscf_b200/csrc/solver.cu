@@ -22,7 +22,6 @@
 #include <stdexcept>
 #include <string>
 #include <thread>
-#include <tuple>
 #include <vector>
 
 #include "../../include/v2rdm_gpu.h"
@@ -335,6 +334,9 @@ struct DeviceTables {
     MapTable<TableBuf> mA, mAT;
     TableBuf<double> b;
     std::vector<double> hb;
+    // the map variants that the autotuner chose, by (A or A^T, instances)
+    std::mutex tuned_mu;
+    std::map<std::pair<int, int>, int> tuned;
     const DevMap& A() const { return mA.dm; }
     const DevMap& AT() const { return mAT.dm; }
     int max_long() const { return std::max(mA.dm.nlong, mAT.dm.nlong); }
@@ -1148,18 +1150,16 @@ class GroupRun {
     // The autotuner of the map kernels: for this group's layout and instance
     // count, every variant of kMapVariants is timed on A and on A^T (CUDA
     // events around a few launches on the group's stream) and the fastest is
-    // kept for the process (the choice depends only on layout and B).
+    // kept with the layout's tables (the choice depends only on layout and B).
     void tune_maps() {
-        static std::mutex mu;
-        static std::map<std::tuple<const void*, int, int>, int> chosen;
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         for (int which = 0; which < 2; which++) {
             DevMap& M = which == 0 ? mA_ : mAT_;
-            const auto key = std::make_tuple((const void*)M.rows, B_, which);
+            const auto key = std::make_pair(which, B_);
             {
-                std::lock_guard<std::mutex> lk(mu);
-                auto it = chosen.find(key);
-                if (it != chosen.end()) {
+                std::lock_guard<std::mutex> lk(T_.tuned_mu);
+                auto it = T_.tuned.find(key);
+                if (it != T_.tuned.end()) {
                     M.variant = it->second;
                     continue;
                 }
@@ -1188,8 +1188,8 @@ class GroupRun {
                 }
             }
             M.variant = bestv;
-            std::lock_guard<std::mutex> lk(mu);
-            chosen[key] = bestv;
+            std::lock_guard<std::mutex> lk(T_.tuned_mu);
+            T_.tuned[key] = bestv;
         }
         if (e0) cudaEventDestroy(e0);
         if (e1) cudaEventDestroy(e1);
