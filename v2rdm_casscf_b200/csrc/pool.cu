@@ -13,6 +13,7 @@ std::mutex g_mu;
 std::map<int, cudaMemPool_t> g_pools;
 std::multimap<size_t, void*> g_pinned;
 size_t g_pinned_bytes = 0;
+int g_owners = 0;
 
 cudaMemPool_t pool_of(int device) {
     std::lock_guard<std::mutex> lk(g_mu);
@@ -128,6 +129,38 @@ void pinned_free(void* p, size_t bytes) {
         }
     }
     cudaFreeHost(p);
+}
+
+size_t pool_idle(int device) {
+    const cudaMemPool_t pool = pool_of(device);
+    unsigned long long reserved = 0, used = 0;
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess || used > reserved)
+        return 0;
+    return reserved - used;
+}
+
+PoolOwner::PoolOwner() {
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_owners++;
+}
+
+PoolOwner::~PoolOwner() {
+    std::map<int, cudaMemPool_t> pools;
+    std::multimap<size_t, void*> pinned;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        if (--g_owners > 0) return;
+        pools = g_pools;
+        pinned.swap(g_pinned);
+        g_pinned_bytes = 0;
+    }
+    for (const auto& b : pinned) cudaFreeHost(b.second);
+    for (const auto& d : pools)
+        if (d.second) on_device(d.first, [&] {
+            cudaStreamSynchronize(cudaStreamLegacy);  // the frees queued there
+            cudaMemPoolTrimTo(d.second, 0);
+        });
 }
 
 }  // namespace v2g

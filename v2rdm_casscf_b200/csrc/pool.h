@@ -14,8 +14,9 @@
 
 namespace v2g {
 
-// Unused bytes the pools keep: device memory per device beyond which it goes
-// back to the system at the next synchronisation, pinned memory in all.
+// Unused bytes the pools keep while a PoolOwner lives: device memory per device
+// beyond which it goes back to the system at the next synchronisation, pinned
+// memory in all.
 constexpr size_t kPoolKeep = size_t(1) << 30;
 constexpr size_t kPinnedKeep = size_t(16) << 20;
 
@@ -30,6 +31,19 @@ void pool_free(void* p, int device);  // device: where it was allocated
 // its owner goes: device_free waits for the device, whatever the stream.
 cudaError_t device_alloc(void** p, size_t bytes);
 void device_free(void* p, int device);
+
+// Device memory that the pool holds unused: it serves the pool's next allocations,
+// beside what the device has free.
+size_t pool_idle(int device);
+
+// Handles and networks own one each; when the last goes, the pools give back all
+// that they hold unused.
+struct PoolOwner {
+    PoolOwner();
+    ~PoolOwner();
+    PoolOwner(const PoolOwner&) = delete;
+    PoolOwner& operator=(const PoolOwner&) = delete;
+};
 
 // Page-locked host memory, in powers of two.  Give back only what no copy in
 // flight uses.

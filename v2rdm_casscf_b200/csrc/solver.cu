@@ -1759,6 +1759,7 @@ void require_device() {
 using v2g::Problem;
 
 struct v2g_handle {
+    v2g::PoolOwner pool;  // goes last
     Problem P;
 };
 

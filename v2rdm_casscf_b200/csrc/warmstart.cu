@@ -25,6 +25,7 @@
 
 #include "kernels.cuh"
 #include "mlp.h"
+#include "pool.h"
 #include "warmstart.h"
 
 namespace v2g {
@@ -218,6 +219,7 @@ void ws_features(int n, double nalpha, const double* h, const double* L, int nq,
 using v2g::WsNet;
 
 struct v2g_warmstart {
+    v2g::PoolOwner pool;  // goes last
     WsNet net;
     v2g_warmstart(int hidden, int device, unsigned long long seed) : net(hidden, device, seed) {}
 };
