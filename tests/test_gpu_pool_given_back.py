@@ -68,3 +68,17 @@ s = project(18)
 del s
 assert before - free() <= 16 * MB, before - free()
 """)
+
+
+def test_anderson_history_beside_held_memory(v2g):
+    # the history of one n = 14 instance takes 0.13 GiB of the 0.5 that the pool holds
+    r = run("""
+keep = V.V2RDMSolver([2], 1, 1)
+hold()
+s = V.V2RDMSolver.from_active_space(synthetic(14, 1), start="feasible", projection="adaptive", anderson_memory=10,
+                                    options=dict(MAXITER=2))
+s.update_xz(1.0)
+block = fill(100 * MB)
+assert V.solve_batch([s])[0]["oiter"] == 2
+""")
+    assert "Anderson" not in r.stderr

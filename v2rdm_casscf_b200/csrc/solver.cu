@@ -953,13 +953,15 @@ class GroupRun {
     }
 
     // The Anderson history of the group (after every other buffer): (3 + 2 m)
-    // state vectors.  m shrinks to what 80 % of the free device memory holds,
+    // state vectors.  m shrinks to what 80 % of the free device memory holds (what
+    // the pool holds unused is free here: the history is allocated from it first),
     // or the acceleration is switched off for this group, with a note on stderr.
     void alloc_anderson(size_t X) {
         for (auto* p : P_) aa_m_ = std::max(aa_m_, p->opt.anderson_memory);
         if (aa_m_ <= 0) return;
         size_t free_b = 0, total_b = 0;
         CK(cudaMemGetInfo(&free_b, &total_b));
+        free_b += pool_idle(T_.device);
         const double vec = 2.0 * (double)X * sizeof(double);
         const int fit = (int)std::floor((0.8 * (double)free_b / vec - 3.0) / 2.0);
         if (fit < aa_m_) {
