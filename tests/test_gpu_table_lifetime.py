@@ -84,3 +84,24 @@ def test_projections_after_their_handle(v2g):
     others(v2g)
     side.synchronize()
     assert np.array_equal(want[0], x.cpu().numpy()) and np.array_equal(want[1], z.cpu().numpy())
+
+
+@pytest.mark.parametrize("n", [4, 8, 12, 16])
+def test_first_map_on_a_side_stream(v2g, n):
+    """The tables are on the device before a caller's stream reads them: the
+    first application of a layout is a handle's first call, on a stream that
+    waits for no other."""
+    import torch
+
+    from helpers import csr_of
+
+    s = v2g.V2RDMSolver([n], n // 2, n // 2, options=dict(CONSTRAIN_SPIN=n != 12))
+    A = csr_of(s)
+    y = np.random.default_rng(n).standard_normal(s.nconstraints)
+    d_in, d_out = torch.from_numpy(y).cuda(), torch.empty(s.dimx, dtype=torch.float64, device="cuda")
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    s.map_batched_device(1, d_in.data_ptr(), d_out.data_ptr(), side.cuda_stream, transpose=True)
+    side.synchronize()
+    want = A.T @ y
+    assert np.abs(d_out.cpu().numpy() - want).max() <= 1e-12 * np.abs(want).max()

@@ -375,6 +375,9 @@ std::shared_ptr<DeviceTables> get_tables(const Layout& L, int device) {
     T->mAT.build(AT);
     build_b(L, T->hb);
     T->b.upload(T->hb.data(), T->hb.size());
+    // a copy from pageable memory may return before its last part has arrived, and
+    // a caller's non-blocking stream does not wait for it
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
     g_cache[key] = T;
     return T;
 }
