@@ -143,7 +143,8 @@ int cg_loop_grid(int device);
 size_t cg_loop_slots(int grid, int B);
 // The whole solve from y, rhs and cs (tol, active, maxiter set): iterates
 // until no instance is active or cap iterations; y, r, p, q and cs as the
-// launches above leave them; *n_active the instances still active, *iters the
+// launches above leave them, but p where the resident kernel runs, which keeps it
+// in registers; *n_active the instances still active, *iters the
 // iterations run, *err = 1 if a wait of the grid's exchanges ran out
 // (then the results are invalid; *err must be 0 at the launch).  slots holds
 // cg_loop_slots(grid, B) words.

@@ -18,8 +18,13 @@ namespace v2g {
 constexpr int kMaxBuckets = 7;
 constexpr int kBucketWidths[kMaxBuckets] = {1, 2, 4, 5, 8, 16, 32};
 constexpr int kMidRow = 256, kMidMany = 32;
-// maps with fewer rows are bound by latency at small batches: their rows of 17
-// to 32 entries take a warp each too, instead of one thread
+// Maps with fewer rows are bound by latency at small batches: their rows of 17 to
+// 32 entries take a warp each too, instead of one thread.  The table is built once
+// for every number of instances, and this is the better side at few of them (B200,
+// us for A / A^T, warp and thread: n = 6 with T1, one instance 2.4 / 2.9 and 2.3 /
+// 3.6; n = 7, four 3.2 / 3.9 and 3.5 / 4.8; n = 12 DG, one 3.3 / 3.7 and 3.3 /
+// 5.5), the other one from sixteen on (n = 5, 64 instances 7.6 / 7.0 and 3.6 / 4.4;
+// n = 7, 32 8.3 / 9.4 and 6.8 / 5.2; n = 12 DG, 128 81 / 93 and 82 / 88).
 constexpr int kLatencyRows = 1 << 18;
 
 // The bucket of a row of len entries in a map of nrows rows; kMaxBuckets: a

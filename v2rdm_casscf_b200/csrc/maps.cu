@@ -31,8 +31,10 @@ inline int grid_for(int64_t work, int threads = kThreads) {
 
 constexpr int kRedBlocks = 148 * 4;
 constexpr int kSpmvBlocks = 148 * 64;
-// resident CTAs of the map kernels (64 registers a thread; three CTAs with 80
-// registers: 334 us where four took 319, n = 20, 19 instances)
+// resident CTAs of the map kernels: 64 registers a thread.  Measured with the bare
+// store alone (three CTAs with 80 registers: 334 us where four took 319, n = 20,
+// 19 instances); the CG's epilogues with two instances per lane spill 200 to 560
+// bytes a thread at 64 registers and were not measured with more.
 constexpr int kMapCtasPerSm = 4;
 
 // Thread mapping shared by the map and vector kernels that also reduce: the
@@ -100,9 +102,10 @@ __device__ __forceinline__ double cta_instance_sum(double v, int B) {
 // instance, beside the launch) and, in a batch, that latency against the loads
 // in flight.  In the deep form a thread works on several rows at once, a pass
 // of blockDim / lanes rows apart, with eight gathers in flight, and loads the
-// table entries of its next tile meanwhile.  The sum of a row runs in slot
-// order in one thread, whatever the form.  A and A^T one after the other on a
-// B200, before and now:
+// table entries of its next tile meanwhile.  The sum of a row of a bucket runs in
+// slot order in one thread, whatever the form; mid and long rows are summed by
+// several threads and folded in a fixed order.  A and A^T one after the other on
+// a B200, before and now:
 //   n = 20, 19 instances   706 -> 275 us   (1.3 -> 3.4 TB/s of vector bytes)
 //   n = 28, 1 instance     243 ->  83 us
 //   n = 8 T2, 3 instances   99 ->  37 us
@@ -1313,8 +1316,9 @@ __global__ void __launch_bounds__(ONE ? kResThreads : 768, 1) cg_resident_kernel
 
 }  // namespace
 
-// Whether table loads and output stores bypass the caches (streaming hints):
-// the autotuner's choice, or streamed from eight instances up.
+// Whether the deep form's table loads and output stores bypass the caches
+// (streaming hints): the autotuner's choice, or streamed from eight instances up.
+// The plain form has no such variant.
 static bool map_streamed(const DevMap& M, int B) {
     if (M.variant >= 0 && M.variant < kMapVariants) return M.variant == 1;
     return B >= 8;

@@ -1469,7 +1469,9 @@ class GroupRun {
     // / 0.61, n = 13 four 1.5 / 3.8, n = 20 one 3.2 / 5.7, n = 24 one 8.4 /
     // 9.4 (2.6e9 = sum of n^3), n = 28 one 20 / 18; many blocks: n = 14 twelve
     // instances 8.3 / 9.2 (1.2e9), n = 10 a hundred 11.7 / 10.9 (1.3e9).
-    // Exact projections: n = 10 one 0.33 / 3.3, n = 20 one 4.4 / 18.7.
+    // Exact projections: n = 10 one 0.29 / 3.7, n = 20 one 3.7 / 19.8, n = 20 four
+    // (3.4e9) 12.3 / 36.7, n = 28 one (6.5e9) 20.6 / 65.8, n = 14 twelve 7.8 / 20.5,
+    // n = 10 forty 4.1 / 11.1: no end to the sign's side in sight at their limit.
     bool use_sign() const {
         const int grid = sign_grid(T_.device);
         if (grid <= 0) return false;
