@@ -85,9 +85,11 @@ int64_t bucket_tiles(const Map& M, int i, int64_t rpp, bool deep) {
 // one latency chain, and more CTAs spread it wider).
 template <class Map>
 bool wants_deep(const Map& M, int B, int threads, int deep_from) {
+    if (!M.packed) return false;
+    const int64_t rpp = threads / lanes_of(B);
     int64_t tot = 0;
-    for (int i = 0; i < M.nb; i++) tot += bucket_tiles(M, i, threads / lanes_of(B), false);
-    return M.packed && tot > deep_from;
+    for (int i = 0; i < M.nb; i++) tot += bucket_tiles(M, i, rpp, false);
+    return tot > deep_from;
 }
 
 // The units of a map in the given form, which has to be the kernel's.
@@ -96,11 +98,12 @@ Blocks map_blocks(const Map& M, int B, int threads, bool deep) {
     Blocks bl{};
     bl.mid = M.nlong - M.nmid;
     bl.midchunks = (B + 31) / 32;
+    const int64_t rpp = threads / lanes_of(B);
     const int warps = threads / 32;
     int acc = bl.mid + (M.nmid + warps - 1) / warps * bl.midchunks;
     for (int i = 0; i < M.nb; i++) {
         bl.start[i] = acc;
-        acc += (int)bucket_tiles(M, i, threads / lanes_of(B), deep);
+        acc += (int)bucket_tiles(M, i, rpp, deep);
     }
     for (int i = M.nb; i <= kMaxBuckets; i++) bl.start[i] = acc;
     return bl;
