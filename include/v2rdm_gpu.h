@@ -162,7 +162,8 @@ int v2g_apply_AT_device(v2g_handle* h, const double* d_u, double* d_out);
 
 /* The maps applied to nvec vectors at once, stored instance-interleaved on
  * the device (element e of vector v at [e * nvec + v], 1 <= nvec <= 256), on
- * the given CUDA stream (NULL: the legacy default stream).  Asynchronous. */
+ * the given CUDA stream (NULL: the legacy default stream), on any 8-byte
+ * boundary.  Asynchronous; v2g_destroy waits for what is queued. */
 int v2g_apply_A_batched_device(v2g_handle* h, int nvec, const double* d_u, double* d_out, void* stream);
 int v2g_apply_AT_batched_device(v2g_handle* h, int nvec, const double* d_u, double* d_out, void* stream);
 

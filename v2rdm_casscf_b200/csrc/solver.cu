@@ -2323,7 +2323,7 @@ int v2g_export_A(v2g_handle* h, long* rowptr, int* col, double* val) {
 // allocations, programs that run under a fixed device-memory budget, and
 // callers that must not take the implicit device synchronisation a
 // cudaMalloc/cudaFree can cause.  v2g_update_xz_noalloc serves them for
-// layouts whose blocks all take the shared-memory eigensolver (dimension
+// layouts whose blocks all fit one CTA's shared memory (dimension
 // <= 64).  Its scratch, the A^T y intermediate, the block task list and mu,
 // lives in the file-scope array below: every GPU that loads this library
 // holds it until the process exits, and every call shares it.
